@@ -116,15 +116,20 @@ def _weights(g, N, K, bf16=False):
     return w.to(torch.bfloat16) if bf16 else w
 
 
+def _operands(g, case):
+    """fp8 operands and their scales, in the operator's layouts."""
+    M, N, K = case["M"], case["N"], case["K"]
+    n_total = case.get("n_total") or N
+    return {"A": _fp8(g, M * K), "B": _fp8(g, N * K), "a_scale": _scales(g, M * (K // 128)),
+            "b_scale": _scales(g, (n_total + 127) // 128 * (K // 128))}
+
+
 def prepare(case, seed):
     g = _gen(seed)
     op, M, K = case["op"], case["M"], case["K"]
     state = {"case": case}
     if op == "gemm":
-        N = case["N"]
-        n_total = case.get("n_total") or N
-        state.update(A=_fp8(g, M * K), B=_fp8(g, N * K), a_scale=_scales(g, M * (K // 128)),
-                     b_scale=_scales(g, (n_total + 127) // 128 * (K // 128)), n0=case.get("n0") or 0, n_total=n_total)
+        state.update(_operands(g, case), n0=case.get("n0") or 0, n_total=case.get("n_total") or case["N"])
     elif op == "linear":
         Wq, Ws = f.quantize_block(_weights(g, case["N"], K, case["bf16"]))
         state.update(X=_activations(g, M, K, case["bf16"]), Wq=Wq, Ws=Ws)
@@ -136,12 +141,11 @@ def prepare(case, seed):
         state["src"] = torch.where(q == 0, q, q + 8)
     else:
         # operands and result in the program's own pinned buffers, as numpy arrays; the context is kept between calls
-        N, sn = case["N"], (case["N"] + 127) // 128
+        N = case["N"]
         state["ctx"] = f.HostContext(M, N, K)
         state["C_host"] = torch.empty(M, N, dtype=torch.bfloat16, pin_memory=True)
         state["C"] = state["C_host"].view(torch.int16).numpy()
-        for name, values in (("A", _fp8(g, M * K)), ("B", _fp8(g, N * K)), ("a_scale", _scales(g, M * (K // 128))),
-                             ("b_scale", _scales(g, sn * (K // 128)))):
+        for name, values in _operands(g, case).items():
             state[name] = values.cpu().pin_memory().numpy()
     return state
 
@@ -186,3 +190,43 @@ def tolerance(case):
     # bf16 results of fp32 sums.  The rounding to bf16 alone is 1.66e-3 (2-norm) and 3.9e-3 at most (against float64);
     # four times that.
     return {"rel": 6.6e-3, "max": 1.6e-2}
+
+
+# ------------------------------------------------------- the same results in 64 bits ------------------------------
+def _quantized(X, rows_per_group):
+    """X in groups of rows_per_group rows x 128 columns: the fp8 values and the inverse scale of every group, both as
+    float64.  The quantisation is defined in fp32: scale = (1 / absmax) * 448, value = e4m3(x * scale)."""
+    R, K = X.shape
+    pad = -R % rows_per_group
+    x = torch.nn.functional.pad(X.float(), (0, 0, 0, pad)).view((R + pad) // rows_per_group, rows_per_group, K // 128, 128)
+    scale = x.abs().amax(dim=(1, 3), keepdim=True).clamp(min=1e-12).reciprocal() * 448.0
+    q = (x * scale).clamp(-448.0, 448.0).to(torch.float8_e4m3fn).double().view(R + pad, K)[:R]
+    return q, (1.0 / scale).double().view(-1, K // 128)
+
+
+def _blockwise_product(A, B, a_scale, b_scale):
+    """A [M, K], B [N, K] with scales per row (or column) and 128 k: [M, K / 128], [N, K / 128].  All float64."""
+    return (A * a_scale.repeat_interleave(128, 1)) @ (B * b_scale.repeat_interleave(128, 1)).T
+
+
+def exact(case, seed):
+    g = _gen(seed)
+    op, M, K = case["op"], case["M"], case["K"]
+    if op == "reencode":                                  # bytes and a count
+        return None
+    if op == "quantize":                                  # bytes, and the inverse scales
+        X = _weights(g, M, K, case["bf16"]) if case["kind"] == "block" else _activations(g, M, K, case["bf16"])
+        _, inv = _quantized(X, 128 if case["kind"] == "block" else 1)
+        return None, inv.T.contiguous().flatten()
+    N = case["N"]
+    if op == "linear":
+        Bv, bs = _quantized(_weights(g, N, K, case["bf16"]), 128)
+        Av, as_ = _quantized(_activations(g, M, K, case["bf16"]), 1)
+        return _blockwise_product(Av, Bv, as_, bs.repeat_interleave(128, 0)[:N])
+    t = _operands(g, case)
+    n0 = case.get("n0") or 0
+    A = t["A"].view(torch.float8_e4m3fn).double().view(K, M).T
+    B = t["B"].view(torch.float8_e4m3fn).double().view(K, N).T
+    bs = t["b_scale"].double().view(K // 128, -1).T.repeat_interleave(128, 0)[n0:n0 + N]
+    C = _blockwise_product(A, B, t["a_scale"].double().view(K // 128, M).T, bs)
+    return C if op == "gemm" else C.cpu()
