@@ -47,6 +47,7 @@
 //              promotion warps never wait on a global load (mn_large.hip:50-55 stages the
 //              pre-multiplied scales in LDS for the same reason) and pay one barrier round trip
 //              per 8 K blocks.
+//   (Each of these roles is one thread, chosen by elect.sync, see ptx::elect_one.)
 //   warp 3     idle (completes the warpgroup that gives up its registers).
 //   warps 4..  promotion + epilogue.  TMEM lane = C row, so a thread owns one row and 128
 //              columns; per K block it reads the partial sums with tcgen05.ld, 64 columns at a
@@ -236,7 +237,7 @@ struct FloatCols {
 };
 
 // Converts 64 columns of this thread's row to bf16 (round to nearest even) into a 32-row x 128-byte staging
-// box laid out as the 128-byte-swizzled TMA store expects; then the warp's lane 0 issues the store.
+// box laid out as the 128-byte-swizzled TMA store expects; then one lane issues the store.
 // The box covers rows [row0, row0 + 32) and columns [col, col + 64); lane = row within the box.
 // PENDING: how many of this thread's most recent stores may still be reading shared memory (1 when the warp
 // alternates between two boxes: only the store before the last one used this box); negative: the caller has waited.
@@ -262,23 +263,22 @@ __device__ __forceinline__ void stage_and_store_64(const CUtensorMap* tmC, int n
                                                    int lane, const Cols cols, int col, int row0, int M, int N)
 {
     if constexpr (PENDING >= 0) {
-        if (lane == 0) ptx::tma_store_wait_read<PENDING>();  // the previous store out of this box has read it
+        if (ptx::elect_one()) ptx::tma_store_wait_read<PENDING>();  // the previous store out of this box has read it
         __syncwarp();
     }
     stage_64(stg, lane, cols);
     ptx::fence_proxy_async_smem();
     __syncwarp();
-    if (lane == 0 && col < N && row0 < M) {
+    if (col < N && row0 < M && ptx::elect_one()) {
         // rows >= M and columns >= N are clipped by the hardware; one bulk group covers every destination's copy
         for (int d = 0; d < n_dest; ++d) ptx::tma_store_2d(tmC + d, stg_addr, col, row0);
         ptx::tma_store_commit();
     }
 }
 
-// The two 64-column boxes of a warp's 32 x 128 piece at once: both are staged, then lanes 0 and 1 issue one store each
-// in the same instruction, so the warp pays the issue latency of a TMA store once per tile instead of twice (1-3 % on
-// the shapes with many tiles per CTA).  Bulk groups belong to the issuing thread: lane h issues, and waits for, the
-// stores out of box h.  The caller has made sure that both boxes are free (wait_read<0> in lanes 0 and 1).
+// The two 64-column boxes of a warp's 32 x 128 piece at once: both are staged, then both stores are issued, in one bulk
+// group.  Bulk groups belong to the issuing thread, which elect.sync makes the same one everywhere in a warp.  The
+// caller has made sure that both boxes are free (wait_read<0> in that thread).
 template <class Cols0, class Cols1>
 __device__ __forceinline__ void stage_and_store_2x64(const CUtensorMap* tmC, int n_dest, uint8_t* stg, uint32_t stg_addr,
                                                      int lane, const Cols0 c0, const Cols1 c1, int col, int row0, int M, int N)
@@ -287,9 +287,11 @@ __device__ __forceinline__ void stage_and_store_2x64(const CUtensorMap* tmC, int
     stage_64(stg + 4096, lane, c1);
     ptx::fence_proxy_async_smem();
     __syncwarp();
-    const int mycol = col + lane * 64;
-    if (lane < 2 && mycol < N && row0 < M) {
-        for (int d = 0; d < n_dest; ++d) ptx::tma_store_2d(tmC + d, stg_addr + lane * 4096, mycol, row0);
+    if (col < N && row0 < M && ptx::elect_one()) {
+        for (int d = 0; d < n_dest; ++d) {
+            ptx::tma_store_2d(tmC + d, stg_addr, col, row0);
+            if (col + 64 < N) ptx::tma_store_2d(tmC + d, stg_addr + 4096, col + 64, row0);
+        }
         ptx::tma_store_commit();
     }
 }
@@ -357,7 +359,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     auto sfull_bar = [&](int i) { return bar_base + 8u * (2 * STAGES + 2 * NBUF + i); };
     auto sempty_bar = [&](int i) { return bar_base + 8u * (2 * STAGES + 2 * NBUF + SRING + i); };
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);   // uniform, and known to be
     const int lane = threadIdx.x & 31;
     PROF_CLK0();
     if (threadIdx.x == 0) { PROF_STAMP(8); }
@@ -455,7 +457,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
     if (warp < 4) {
         ptx::setmaxnreg_dec<64>();
-        if (warp == 0 && lane == 0) {
+        if (warp == 0 && ptx::elect_one()) {
             // ---------------------------------------------------- TMA producer: A and B ----
             uint32_t it = 0;
             bool ok = true;
@@ -498,7 +500,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 const long long t0 = clock64();
                 while (clock64() - t0 < 2000000LL) __nanosleep(1000);
             }
-        } else if (warp == 1 && lane == 0 && rank == 0) {
+        } else if (warp == 1 && rank == 0 && ptx::elect_one()) {
             // ---------------------------------------------------- MMA issuer ----------------
             constexpr uint32_t idesc = ptx::make_idesc_e4m3_mnmajor(Cfg::TILE_M, BN);
             uint32_t it = 0, ait = 0, tcount = 0;
@@ -565,7 +567,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             t_mma_total = clock64() - mma_start;
 #endif
             PROF_OUT(1, w_tempty); PROF_OUT(2, w_full); PROF_OUT(3, t_mma_total); PROF_STAMP(11);
-        } else if (warp == 2 && lane == 0) {
+        } else if (warp == 2 && ptx::elect_one()) {
             // ---------------------------------------------------- TMA producer: a_scale ----
             uint32_t sit = 0;
             bool ok = true;
@@ -667,8 +669,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 const float s0l = as0 * bl0, s0h = as0 * bh0, s1l = as1 * bl1, s1h = as1 * bh1;
                 const unsigned long long s0l2 = pack_f32x2(s0l, s0l), s0h2 = pack_f32x2(s0h, s0h);
                 const unsigned long long s1l2 = pack_f32x2(s1l, s1l), s1h2 = pack_f32x2(s1h, s1h);
-                // box h belongs to lane h: its previous store has read the box before anything is staged into it
-                if (lane < 2) ptx::tma_store_wait_read<0>();
+                // the previous stores have read both boxes before anything is staged into them
+                if (ptx::elect_one()) ptx::tma_store_wait_read<0>();
                 ok = wait_bounded(tfull_bar(0), tcount & 1u, abort_flag, p.status, DS_TIMEOUT_TMEM_FULL);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
@@ -706,10 +708,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 if (!last_unit) {
                     ptx::fence_proxy_async_smem();
                     __syncwarp();
-                    const int mycol = ncol0 + lane * 64;
-                    if (lane < 2 && mycol < p.N && m0 + quarter * 32 < p.M) {
-                        for (int d = 0; d < p.n_dest; ++d)
-                            ptx::tma_store_2d(cmaps.m + d, my_stg_addr + lane * 4096, mycol, m0 + quarter * 32);
+                    if (ncol0 < p.N && m0 + quarter * 32 < p.M && ptx::elect_one()) {
+                        for (int d = 0; d < p.n_dest; ++d) {
+                            ptx::tma_store_2d(cmaps.m + d, my_stg_addr, ncol0, m0 + quarter * 32);
+                            if (ncol0 + 64 < p.N) ptx::tma_store_2d(cmaps.m + d, my_stg_addr + 4096, ncol0 + 64, m0 + quarter * 32);
+                        }
                         ptx::tma_store_commit();
                     }
                 }
@@ -804,8 +807,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             // ---- epilogue of a finished tile: fp32 -> bf16 (round to nearest even), staged, TMA store ----
             auto store_tile = [&]() {
                 if constexpr (Cfg::NSTG == 2) {
-                    // box h belongs to lane h: its previous store has read the box before anything is staged into it
-                    if (lane < 2) ptx::tma_store_wait_read<0>();
+                    // the previous stores have read both boxes before anything is staged into them
+                    if (ptx::elect_one()) ptx::tma_store_wait_read<0>();
                     __syncwarp();
                     if (u + unit_step < units) {
                         stage_and_store_2x64(cmaps.m, p.n_dest, my_stg, my_stg_addr, lane, PackedCols{acc[0], acc[1]},
@@ -985,7 +988,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         if (pw == 0 && lane == 0) { PROF_OUT(4, w_sfull); PROF_OUT(5, w_tfull); PROF_OUT(6, t_fma); PROF_OUT(7, t_epi); PROF_STAMP(13); }
 #endif
         // C must have been read out of shared memory before the CTA goes away
-        if (lane < 2) ptx::tma_store_wait_read<0>();
+        if (ptx::elect_one()) ptx::tma_store_wait_read<0>();
         __syncwarp();
     }
 

