@@ -393,23 +393,6 @@ static int encode_operand_map(CUtensorMap* tm, const void* base, int mn, int K)
     return FP8BS_OK;
 }
 
-// a_scale as a 2-D fp32 tensor {M, K/128}; one box = the scales of a tile's 128 rows for SCALE_GROUP K blocks.
-static int encode_scale_map(CUtensorMap* tm, const float* base, int M, int KB)
-{
-    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(M), static_cast<cuuint64_t>(KB)};
-    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(M) * 4};
-    const cuuint32_t box[2] = {128u, static_cast<cuuint32_t>(SCALE_GROUP)};
-    const cuuint32_t estr[2] = {1u, 1u};
-    const CUresult r = g_encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides,
-                                      box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS) {
-        tl_last_cuda_error = static_cast<int>(r);
-        return FP8BS_ERR_CUDA;
-    }
-    return FP8BS_OK;
-}
-
 // C as a 2-D bf16 tensor {N, M} (row-major M x N); a store box is 64 columns x 32 rows, 128-byte swizzled.
 static int encode_c_map(CUtensorMap* tm, void* base, int M, int N, int ld)
 {
@@ -429,7 +412,7 @@ static int encode_c_map(CUtensorMap* tm, void* base, int M, int N, int ld)
 }
 
 struct TensorMaps {
-    CUtensorMap A, B, As;
+    CUtensorMap A, B;
     CMaps C;
 };
 
@@ -457,7 +440,7 @@ static int launch(const TensorMaps& tm, const GemmParams& p, int sm_count, cudaS
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = g_use_pdl ? 2 : 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_kernel<BN, CG, MODE>, tm.A, tm.B, tm.As, tm.C, p);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_kernel<BN, CG, MODE>, tm.A, tm.B, tm.C, p);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     CUDA_TRY(e);
     return FP8BS_OK;
@@ -523,13 +506,13 @@ static int gemm_impl(const void* A, const void* B, const float* a_scale, const f
     TensorMaps tm{};
     if ((rc = encode_operand_map(&tm.A, A, M, K))) return rc;
     if ((rc = encode_operand_map(&tm.B, B, N, K))) return rc;
-    if ((rc = encode_scale_map(&tm.As, a_scale, M, K / 128))) return rc;
     if (dests) {
         for (int d = 0; d < n_dest; ++d)
             if ((rc = encode_c_map(&tm.C.m[d], static_cast<__nv_bfloat16*>(dests[d]) + n0, M, N, n_total))) return rc;
     } else if ((rc = encode_c_map(&tm.C.m[0], C, M, N, N))) return rc;
 
     GemmParams p;
+    p.a_scale = a_scale;
     p.b_scale = b_scale;
     p.C = static_cast<__nv_bfloat16*>(C);
     p.partials = nullptr;

@@ -43,11 +43,13 @@
 //              fresh TMEM buffer (the first one overwrites), then a commit that publishes the TMEM
 //              buffer and, in the three-stage kernels, a second one that frees the shared-memory stage
 //              (with four or more stages a promotion warp frees it, see PROMO_RELEASE).
-//   warp 2     TMA producer for a_scale: boxes of 128 rows x 8 K blocks into a small ring, so the
-//              promotion warps never wait on a global load (mn_large.hip:50-55 stages the
-//              pre-multiplied scales in LDS for the same reason) and pay one barrier round trip
-//              per 8 K blocks.
 //   (Each of these roles is one thread, chosen by elect.sync, see ptx::elect_one.)
+//   warp 2     scale products: a_scale * b_scale of the tile's rows and 64-column pieces into shared memory, one slot
+//              per K block (the reference stages the pre-multiplied scales in LDS too, mn_large.hip:50-55).  The promotion
+//              warps get slot and partial sums through one barrier and read a K block's scales with one shared-memory
+//              load; when they made the products themselves (an a_scale ring with barriers of its own, b_scale by
+//              shuffles) they spent ~400 of ~850 cycles per K block on that, with the tensor pipe waiting.  Measured:
+//              6144 x 4608 x 7168 182 -> 168 us, 6144 x 4096 x 512 22.4 -> 20.7, 1024 x 3072 x 1536 11.0 -> 10.5.
 //   warp 3     idle (completes the warpgroup that gives up its registers).
 //   warps 4..  promotion + epilogue.  TMEM lane = C row, so a thread owns one row and 128
 //              columns; per K block it reads the partial sums with tcgen05.ld, 64 columns at a
@@ -74,8 +76,7 @@ enum : uint32_t {
     DS_TIMEOUT_STAGE_FULL = 2,   // MMA warp waited for TMA data
     DS_TIMEOUT_TMEM_EMPTY = 3,   // MMA warp waited for the promotion warps
     DS_TIMEOUT_TMEM_FULL = 4,    // promotion warps waited for the MMA warp
-    DS_TIMEOUT_SCALE_EMPTY = 5,  // scale producer waited for the promotion warps
-    DS_TIMEOUT_SCALE_FULL = 6,   // promotion warps waited for a_scale
+    DS_TIMEOUT_SCALE_EMPTY = 5,  // scale warp waited for an earlier K block's hand-over
 };
 
 // Where a finished C tile goes: the caller's C, and for the fused distribution (fp8bs_gemm_scatter) the same window
@@ -86,6 +87,7 @@ struct CMaps {
 };
 
 struct GemmParams {
+    const float* a_scale;    // [M, K/128], m contiguous            (check.cu:45)
     const float* b_scale;    // [sn, K/128], nb contiguous          (check.cu:46)
     __nv_bfloat16* C;        // M x N row-major                     (check.cu:48)
     float4* partials;        // split-K only: [half-tile][split][BN/4][128] float4
@@ -102,11 +104,6 @@ struct GemmParams {
     long long* prof;         // per CTA: 8 cycle counters (profiling builds only)
 #endif
 };
-
-// a_scale reaches shared memory in boxes of 128 rows x SCALE_GROUP K blocks (the tensor map's box, see the host side):
-// one barrier round trip per SCALE_GROUP K blocks instead of one per block.  Measured on B200 with the promotion loop
-// otherwise unchanged: a per-block hand-off cost ~160 cycles per K block of a loop that has ~512 to spend.
-constexpr int SCALE_GROUP = 8;
 
 template <int BN, int CG>
 struct TileCfg {
@@ -131,14 +128,15 @@ struct TileCfg {
     // than with one box and 5 stages at every K.
     static constexpr int NSTG = COLS / 64;
     static constexpr int STG_BYTES = PROMO_WARPS * 4096 * NSTG;
-    static constexpr int SGRP = SCALE_GROUP;          // K blocks per a_scale ring entry (one TMA box {128 rows, SGRP})
-    static constexpr int SRING = 4;                   // a_scale ring entries
-    static constexpr int SRING_BYTES = SRING * SGRP * 512;
+    static constexpr int QUADS = COLS / 64;           // 64-column pieces per promotion thread, one scale product each
+    static constexpr int SSLOTS = 2 * NBUF;           // scale-product slots, one per K block in flight
+    static constexpr int SSLOT_FLOATS = 2 * 128 * QUADS;   // [column group][row][piece]
+    static constexpr int SRING_BYTES = SSLOTS * SSLOT_FLOATS * 4;
     static constexpr int SMEM_LIMIT = 232448;         // 227 KB per CTA
     static constexpr int FIXED = 1024 + STG_BYTES + SRING_BYTES + 512;
     static constexpr int STAGES = (SMEM_LIMIT - FIXED) / STAGE_BYTES;
     static_assert(STAGES >= 2, "pipeline depth");
-    static constexpr int NUM_BARS = 2 * STAGES + 2 * NBUF + 2 * SRING;
+    static constexpr int NUM_BARS = 2 * STAGES + 2 * NBUF;
     static_assert(NUM_BARS * 8 + 64 <= 512, "barrier area");
     static constexpr int SMEM_BYTES = FIXED + STAGES * STAGE_BYTES;
 };
@@ -148,13 +146,13 @@ constexpr long long WAIT_LIMIT_CYCLES = 2000000000LL;  // about one second
 // Instrumentation, compiled in only by `python -m fp8_quant_matmul_b200.build --profile[=LEVEL]` (-DFP8BS_PROFILE=LEVEL,
 // into a separate libfp8bs_prof.so).  Layout of the buffer GemmParams::prof points to, in 64-bit words:
 //   [cta * 16 + slot]           slots 0-7 cycle counters (level >= 2): producer wait for a free stage, MMA wait for a
-//                               free TMEM buffer, MMA wait for operands, MMA loop total, promotion wait for a_scale,
+//                               free TMEM buffer, MMA wait for operands, MMA loop total, not used,
 //                               promotion wait for partial sums, promotion loads + FMAs, epilogue;
 //                               slots 8-14 %globaltimer stamps in ns: kernel start, set-up done, first operands
 //                               there, MMA loop done, promotion loop done, all stores issued, exit; slot 15 the
 //                               CTA's lifetime in cycles
 //   [4096 + event * 128 + kb]   level 3, CTA 0, first 128 K blocks, clock64 at: 0 TMEM buffer free (MMA warp),
-//                               1 operands there, 2 MMAs and commits issued, 3 a_scale there (promotion warp 4),
+//                               1 operands there, 2 MMAs and commits issued, 3 not used,
 //                               4 partial sums there, 5 FMAs done, 6 stage free (producer), 7 / 8 = 4 / 5 for warp 5;
 //                               [4096 + (9 or 10) * 128 + unit]: start / end of the epilogue of CTA 0's unit
 #ifdef FP8BS_PROFILE
@@ -317,12 +315,11 @@ __global__ void wait_timeout_selftest_kernel(unsigned int* status, long long lim
 template <int BN, int CG, int MODE>
 __global__ void __launch_bounds__(TileCfg<BN, CG>::THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-            const __grid_constant__ CUtensorMap tmAs, const __grid_constant__ CMaps cmaps, const GemmParams p)
+            const __grid_constant__ CMaps cmaps, const GemmParams p)
 {
     using Cfg = TileCfg<BN, CG>;
     constexpr int STAGES = Cfg::STAGES;
     constexpr int NBUF = Cfg::NBUF;
-    constexpr int SRING = Cfg::SRING;
     constexpr bool SPLITK = (MODE == 1 || MODE == 2);   // K cut into p.splits equal ranges per tile
     constexpr bool STREAMK = (MODE == 3);               // K blocks of all tiles dealt out evenly, see below
     static_assert(MODE != 2 || CG == 1, "the cluster reduction uses the cluster for the K splits");
@@ -343,11 +340,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     const uint32_t raw = ptx::smem_u32(smem_raw);
     const uint32_t stage_base = (raw + 1023u) & ~1023u;   // swizzle atoms need 1024-byte alignment
     uint8_t* aligned = smem_raw + (stage_base - raw);
-    // layout: [stages][epilogue staging][a_scale ring][barriers + control words]
+    // layout: [stages][epilogue staging][scale products][barriers + control words]
     const uint32_t stg_base = stage_base + STAGES * Cfg::STAGE_BYTES;
     uint8_t* stg_ptr = aligned + STAGES * Cfg::STAGE_BYTES;
     const uint32_t sring_base = stg_base + Cfg::STG_BYTES;
-    const float* sring_ptr = reinterpret_cast<const float*>(stg_ptr + Cfg::STG_BYTES);
+    float* slots_ptr = reinterpret_cast<float*>(stg_ptr + Cfg::STG_BYTES);
     const uint32_t bar_base = sring_base + Cfg::SRING_BYTES;
     volatile uint32_t* ctrl = reinterpret_cast<volatile uint32_t*>(stg_ptr + Cfg::STG_BYTES + Cfg::SRING_BYTES +
                                                                     Cfg::NUM_BARS * 8);
@@ -356,8 +353,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
     auto tfull_bar = [&](int b) { return bar_base + 8u * (2 * STAGES + b); };
     auto tempty_bar = [&](int b) { return bar_base + 8u * (2 * STAGES + NBUF + b); };
-    auto sfull_bar = [&](int i) { return bar_base + 8u * (2 * STAGES + 2 * NBUF + i); };
-    auto sempty_bar = [&](int i) { return bar_base + 8u * (2 * STAGES + 2 * NBUF + SRING + i); };
 
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);   // uniform, and known to be
     const int lane = threadIdx.x & 31;
@@ -370,19 +365,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     if (threadIdx.x == 0) {
         ptx::prefetch_tensormap(&tmA);
         ptx::prefetch_tensormap(&tmB);
-        ptx::prefetch_tensormap(&tmAs);
         for (int d = 0; d < p.n_dest; ++d) ptx::prefetch_tensormap(&cmaps.m[d]);
         for (int s = 0; s < STAGES; ++s) {
             ptx::mbar_init(full_bar(s), 1);
             ptx::mbar_init(empty_bar(s), 1);
         }
         for (int b = 0; b < NBUF; ++b) {
-            ptx::mbar_init(tfull_bar(b), 1);
+            ptx::mbar_init(tfull_bar(b), 2);                         // the MMA warp's commit and the scale warp
             ptx::mbar_init(tempty_bar(b), Cfg::PROMO_WARPS * CG);   // the leader also hears from the peer's warps
-        }
-        for (int i = 0; i < SRING; ++i) {
-            ptx::mbar_init(sfull_bar(i), 1);
-            ptx::mbar_init(sempty_bar(i), Cfg::PROMO_WARPS);
         }
         ctrl[1] = 0u;
         ctrl[2] = 0u;
@@ -459,7 +449,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         ptx::setmaxnreg_dec<64>();
         if (warp == 0 && ptx::elect_one()) {
             // ---------------------------------------------------- TMA producer: A and B ----
-            uint32_t it = 0;
+            uint32_t it = 0, sphase = 0;
+            int stage = 0;
             bool ok = true;
             PROF_DECL(w_empty);
             for (int u = unit0; u < units && ok; u += unit_step) {
@@ -470,8 +461,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 nbox = nbox < 0 ? 0 : (nbox < Cfg::NBOX_B ? nbox : Cfg::NBOX_B);
                 if (CG == 2) nbox = Cfg::NBOX_B;                              // pairs: fixed byte count (zero fill)
                 for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1u;
+                    const int s = stage;
+                    const uint32_t ph = sphase;
+                    if (++stage == STAGES) { stage = 0; sphase ^= 1u; }
                     { PROF_T0();
                     ok = wait_bounded(empty_bar(s), ph ^ 1u, abort_flag, p.status, DS_TIMEOUT_STAGE_EMPTY);
                     PROF_ADD(w_empty); }
@@ -503,7 +495,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         } else if (warp == 1 && rank == 0 && ptx::elect_one()) {
             // ---------------------------------------------------- MMA issuer ----------------
             constexpr uint32_t idesc = ptx::make_idesc_e4m3_mnmajor(Cfg::TILE_M, BN);
-            uint32_t it = 0, ait = 0, tcount = 0;
+            uint32_t it = 0, ait = 0, tcount = 0, sphase = 0;
+            int stage = 0;
             bool ok = true;
             PROF_DECL(w_tempty); PROF_DECL(w_full); PROF_DECL(t_mma_total);
 #ifdef FP8BS_PROFILE
@@ -513,8 +506,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 int tile, m0, n0, kb0, kb1;
                 decode(u, tile, m0, n0, kb0, kb1);
                 for (int kb = kb0; kb < kb1; ++kb, ++it, ++ait) {
-                    const int s = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1u;
+                    const int s = stage;
+                    const uint32_t ph = sphase;
+                    if (++stage == STAGES) { stage = 0; sphase ^= 1u; }
                     // MODE 4: K block j of a tile goes to buffer j; the pair is handed over and taken back once per tile
                     // (barriers tfull / tempty number 0, phase = tile count)
                     const int b = RESIDENT ? (kb - kb0) : static_cast<int>(ait % NBUF);
@@ -567,21 +561,81 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             t_mma_total = clock64() - mma_start;
 #endif
             PROF_OUT(1, w_tempty); PROF_OUT(2, w_full); PROF_OUT(3, t_mma_total); PROF_STAMP(11);
-        } else if (warp == 2 && ptx::elect_one()) {
-            // ---------------------------------------------------- TMA producer: a_scale ----
-            uint32_t sit = 0;
+        } else if (warp == 2) {
+            // ---------------------------------------------------- scale products -----------
+            // a_scale[m, kb] * b_scale[n / 128, kb] for the tile's 128 rows and each 64-column piece of its width (n0 and
+            // n_off are multiples of 64, so a piece has one b_scale), one slot per K block (MODE 4: two slots per tile).
+            // The promotion warps wait for the slot and for the partial sums on the same barrier.  Item i is written
+            // once TMEM-full of item i - NB has completed: its own phase of that barrier has then begun, and the MMAs of item
+            // i - NB were issued after every promotion warp had given back the buffer of item i - 2 NB, and with it the slot
+            // that item i reuses.
+            // The scales are read from global memory SAHEAD K blocks before they are needed.
+            constexpr int NB = RESIDENT ? 1 : NBUF;
+            constexpr int NQ = 2 * Cfg::QUADS;                  // 64-column pieces per tile
+            constexpr int SAHEAD = 4;
+            float av[SAHEAD][4], bv[SAHEAD];                    // rows lane + 32 j; lane q < NQ: b_scale of piece q
+            bool valid[SAHEAD];
+            int fu = unit0, fkb = 0, fkb1 = 0, fm = 0, fnb = 0;
+            auto fetch_unit = [&]() {                           // the reading cursor enters unit fu
+                if (fu < units) {
+                    int tile, m0, n0;
+                    decode(fu, tile, m0, n0, fkb, fkb1);
+                    fm = m0 + lane;
+                    fnb = (p.n_off + n0 + (lane & (NQ - 1)) * 64) >> 7;
+                    fnb = fnb < p.sn ? fnb : p.sn - 1;
+                }
+            };
+            auto fetch = [&](float (&a)[4], float& b, bool& v) {
+                v = fu < units;
+                if (!v) return;
+                const float* ap = p.a_scale + static_cast<size_t>(fkb) * p.M + fm;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) a[j] = (fm + 32 * j < p.M) ? __ldg(ap + 32 * j) : 0.0f;
+                b = __ldg(p.b_scale + static_cast<size_t>(fkb) * p.sn + fnb);
+                if (++fkb == fkb1) {
+                    fu += unit_step;
+                    fetch_unit();
+                }
+            };
+            fetch_unit();
+#pragma unroll
+            for (int d = 0; d < SAHEAD; ++d) fetch(av[d], bv[d], valid[d]);
+            uint32_t item = 0;
+            int kpos = 0;                                       // MODE 4: K block within the tile
             bool ok = true;
-            for (int u = unit0; u < units && ok; u += unit_step) {
-                int tile, m0, n0, kb0, kb1;
-                decode(u, tile, m0, n0, kb0, kb1);
-                for (int kb = kb0; kb < kb1; kb += Cfg::SGRP, ++sit) {
-                    const int i = sit % SRING;
-                    const uint32_t ph = (sit / SRING) & 1u;
-                    ok = wait_bounded(sempty_bar(i), ph ^ 1u, abort_flag, p.status, DS_TIMEOUT_SCALE_EMPTY);
+            while (ok) {
+#pragma unroll
+                for (int d = 0; d < SAHEAD; ++d) {
                     if (!ok) break;
-                    // a whole box is always written and counted: rows >= M and K blocks past the end read as 0
-                    ptx::mbar_arrive_expect_tx(sfull_bar(i), Cfg::SGRP * 512);
-                    ptx::tma_load_2d(sring_base + i * (Cfg::SGRP * 512), &tmAs, m0, kb, sfull_bar(i));
+                    if (!valid[d]) { ok = false; break; }       // no more K blocks
+                    if ((!RESIDENT || kpos == 0) && item >= NB) {
+                        ok = wait_bounded(tfull_bar(item % NB), ((item / NB) - 1u) & 1u, abort_flag, p.status, DS_TIMEOUT_SCALE_EMPTY);
+                        ok = __all_sync(0xffffffffu, ok);
+                        if (!ok) break;
+                    }
+                    const int slot = RESIDENT ? static_cast<int>(2 * (item & 1u)) + kpos : static_cast<int>(item % Cfg::SSLOTS);
+                    float* dst = slots_ptr + slot * Cfg::SSLOT_FLOATS + lane * Cfg::QUADS;
+                    float bs[NQ];
+#pragma unroll
+                    for (int q = 0; q < NQ; ++q) bs[q] = __shfl_sync(0xffffffffu, bv[d], q) * p.elem_scale;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+#pragma unroll
+                        for (int g = 0; g < 2; ++g) {
+                            float* w = dst + (g * 128 + 32 * j) * Cfg::QUADS;
+                            if constexpr (Cfg::QUADS == 2)
+                                *reinterpret_cast<float2*>(w) = make_float2(av[d][j] * bs[2 * g], av[d][j] * bs[2 * g + 1]);
+                            else *w = av[d][j] * bs[g];
+                        }
+                    if (!RESIDENT || kpos == KB - 1) {
+                        __syncwarp();
+                        if (lane == 0) ptx::mbar_arrive(tfull_bar(RESIDENT ? 0 : item % NB));
+                        ++item;
+                        kpos = 0;
+                    } else {
+                        ++kpos;
+                    }
+                    fetch(av[d], bv[d], valid[d]);
                 }
             }
         }
@@ -597,41 +651,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         const uint32_t my_stg_addr = stg_base + pw * 4096 * Cfg::NSTG;
         uint32_t lead_tempty = tempty_bar(0);
         if constexpr (CG == 2) lead_tempty = ptx::mapa(tempty_bar(0), 0);
+        const uint32_t slot_addr = sring_base + static_cast<uint32_t>((grp * 128 + row_in_tile) * Cfg::QUADS * 4);
         uint32_t ait = 0;
-        uint32_t sgit = 0;                       // a_scale ring entries consumed so far
+        uint32_t stage = 0;                      // ait % STAGES
         uint32_t tcount = 0;                     // MODE 4: tiles done by this CTA
         bool ok = true;
-        PROF_DECL(w_sfull); PROF_DECL(w_tfull); PROF_DECL(t_fma); PROF_DECL(t_epi);
-        // b_scale lane vectors of unit u: K blocks kb0 + lane and kb0 + 32 + lane of the one or two 128-column blocks
-        // this thread's columns fall into (same index arithmetic as at the top of the unit loop)
-        float pf_bl = 0.0f, pf_bh = 0.0f, pf_bln = 0.0f, pf_bhn = 0.0f;
-        auto fetch_bscale = [&](int u) {
-            int tile, m0, n0, kb0, kb1;
-            decode(u, tile, m0, n0, kb0, kb1);
-            const int g0 = p.n_off + n0 + grp * Cfg::COLS;
-            int lo = g0 >> 7, hi = (g0 >> 7) + 1;
-            lo = lo < p.sn ? lo : p.sn - 1;
-            hi = hi < p.sn ? hi : p.sn - 1;
-            auto ld = [&](int nb, int kbase) {
-                const int k = kbase + lane;
-                return (k < kb1) ? __ldg(p.b_scale + nb + static_cast<size_t>(k) * p.sn) : 0.0f;
-            };
-            pf_bl = ld(lo, kb0);
-            pf_bh = ld(hi, kb0);
-            pf_bln = ld(lo, kb0 + 32);
-            pf_bhn = ld(hi, kb0 + 32);
-        };
-        if (unit0 < units) fetch_bscale(unit0);
+        PROF_DECL(w_tfull); PROF_DECL(t_fma); PROF_DECL(t_epi);
         for (int u = unit0; u < units; u += unit_step) {
             int tile, m0, n0, kb0, kb1;
             decode(u, tile, m0, n0, kb0, kb1);
             const int ncol0 = n0 + grp * Cfg::COLS;           // first local column of this thread
-            const int gcol0 = p.n_off + ncol0;                // its global column (b_scale index)
-            int nb_lo = gcol0 >> 7, nb_hi = (gcol0 >> 7) + 1;  // a thread's columns touch at most two 128-blocks
-            nb_lo = nb_lo < p.sn ? nb_lo : p.sn - 1;
-            nb_hi = nb_hi < p.sn ? nb_hi : p.sn - 1;
-            const int hi_from = 4 - ((gcol0 & 127) >> 5);     // first 32-col chunk that uses nb_hi
-
             // running sums of this thread's row: 4 chunks of 32 columns, two fp32 per 64-bit register
             unsigned long long acc[Cfg::NCH][16];
 #pragma unroll
@@ -639,36 +668,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 #pragma unroll
                 for (int i = 0; i < 16; ++i) acc[c][i] = 0ull;
 
-            // b_scale is tiny and warp-uniform.  Lane l holds the values of K block (base + l); every 32 blocks
-            // the vector loaded one round earlier takes over, so no iteration waits on a global load.  The first two
-            // vectors of a unit were fetched before the previous unit's epilogue (pf_*), so a tile switch does not
-            // wait on global memory either (measured: 3 % on 1024 x 7168 x 256, neutral elsewhere).
-            const float* bl_ptr = p.b_scale + nb_lo;
-            const float* bh_ptr = p.b_scale + nb_hi;
-            auto load_bvec = [&](const float* ptr, int kbase) {
-                const int k = kbase + lane;
-                return (k < kb1) ? __ldg(ptr + static_cast<size_t>(k) * p.sn) : 0.0f;
-            };
-            float bl_vec = pf_bl, bh_vec = pf_bh, bl_nxt = pf_bln, bh_nxt = pf_bhn;
-
             if constexpr (RESIDENT) {
                 // ---- short K: both K blocks of the tile are in TMEM when the MMA warp hands it over ----
                 const bool two = (kb1 - kb0) > 1;
-                const float bl0 = __shfl_sync(0xffffffffu, bl_vec, 0) * p.elem_scale;
-                const float bh0 = __shfl_sync(0xffffffffu, bh_vec, 0) * p.elem_scale;
-                const float bl1 = __shfl_sync(0xffffffffu, bl_vec, 1) * p.elem_scale;
-                const float bh1 = __shfl_sync(0xffffffffu, bh_vec, 1) * p.elem_scale;
-                if (u + unit_step < units) fetch_bscale(u + unit_step);      // in flight during everything below
-                const int si = sgit % SRING;
-                ok = wait_bounded(sfull_bar(si), (sgit / SRING) & 1u, abort_flag, p.status, DS_TIMEOUT_SCALE_FULL);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                const float as0 = sring_ptr[(si * Cfg::SGRP + 0) * 128 + row_in_tile];   // entry released below
-                const float as1 = sring_ptr[(si * Cfg::SGRP + 1) * 128 + row_in_tile];   // 0 when K = 128 (zero fill)
-                // same arithmetic as the K loop of the other modes: acc = fma(p0, s0, 0), then acc = fma(p1, s1, acc)
-                const float s0l = as0 * bl0, s0h = as0 * bh0, s1l = as1 * bl1, s1h = as1 * bh1;
-                const unsigned long long s0l2 = pack_f32x2(s0l, s0l), s0h2 = pack_f32x2(s0h, s0h);
-                const unsigned long long s1l2 = pack_f32x2(s1l, s1l), s1h2 = pack_f32x2(s1h, s1h);
                 // the previous stores have read both boxes before anything is staged into them
                 if (ptx::elect_one()) ptx::tma_store_wait_read<0>();
                 ok = wait_bounded(tfull_bar(0), tcount & 1u, abort_flag, p.status, DS_TIMEOUT_TMEM_FULL);
@@ -678,6 +680,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                                        static_cast<uint32_t>(grp * Cfg::COLS);
                 const bool last_unit = !(u + unit_step < units);
+                // scale products of this row and the thread's two 64-column pieces, both K blocks; slots 2t and 2t + 1
+                const uint32_t sa = slot_addr + 2u * (tcount & 1u) * (Cfg::SSLOT_FLOATS * 4);
+                float s0[2], s1[2];
+                ptx::ld_shared_v2(sa, s0[0], s0[1]);
+                if (two) ptx::ld_shared_v2(sa + Cfg::SSLOT_FLOATS * 4, s1[0], s1[1]);
+                // same arithmetic as the K loop of the other modes: acc = fma(p0, s0, 0), then acc = fma(p1, s1, acc)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     uint32_t v0[64], v1[64];
@@ -691,11 +699,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                     }
 #pragma unroll
                     for (int i = 0; i < 16; ++i) { acc[0][i] = 0ull; acc[1][i] = 0ull; }
-                    ptx::fma32_from64<0>(acc[0], v0, (2 * h >= hi_from) ? s0h2 : s0l2);
-                    ptx::fma32_from64<32>(acc[1], v0, (2 * h + 1 >= hi_from) ? s0h2 : s0l2);
+                    const unsigned long long s0h = pack_f32x2(s0[h], s0[h]);
+                    ptx::fma32_from64<0>(acc[0], v0, s0h);
+                    ptx::fma32_from64<32>(acc[1], v0, s0h);
                     if (two) {
-                        ptx::fma32_from64<0>(acc[0], v1, (2 * h >= hi_from) ? s1h2 : s1l2);
-                        ptx::fma32_from64<32>(acc[1], v1, (2 * h + 1 >= hi_from) ? s1h2 : s1l2);
+                        const unsigned long long s1h = pack_f32x2(s1[h], s1[h]);
+                        ptx::fma32_from64<0>(acc[0], v1, s1h);
+                        ptx::fma32_from64<32>(acc[1], v1, s1h);
                     }
                     if (last_unit) {
                         // the CTA's last tile: each store leaves as soon as its box is staged (shorter tail)
@@ -716,37 +726,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                         ptx::tma_store_commit();
                     }
                 }
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(sempty_bar(si));
-                ++sgit;
                 ++tcount;
                 continue;                                                     // next tile
             }
             if constexpr (!RESIDENT)
             for (int kb = kb0; kb < kb1 && ok; ++kb, ++ait) {
-                const int kj = (kb - kb0) & 31;
-                if (kj == 0 && kb != kb0) {
-                    bl_vec = bl_nxt;
-                    bh_vec = bh_nxt;
-                    bl_nxt = load_bvec(bl_ptr, kb + 32);
-                    bh_nxt = load_bvec(bh_ptr, kb + 32);
-                }
-                const float bl = __shfl_sync(0xffffffffu, bl_vec, kj) * p.elem_scale;
-                const float bh = __shfl_sync(0xffffffffu, bh_vec, kj) * p.elem_scale;
-                // a_scale of this row and block, from the ring: one entry holds SGRP consecutive K blocks
-                const int kr = (kb - kb0) % Cfg::SGRP;
-                const int si = sgit % SRING;
-                if (kr == 0) {
-                    PROF_T0();
-                    ok = wait_bounded(sfull_bar(si), (sgit / SRING) & 1u, abort_flag, p.status, DS_TIMEOUT_SCALE_FULL);
-                    PROF_ADD(w_sfull);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                }
-                if (pw == 0 && lane == 0) PROF_TRACE(3, ait);
-                const float as = sring_ptr[(si * Cfg::SGRP + kr) * 128 + row_in_tile];   // entry released below
-                const float s_lo = as * bl, s_hi = as * bh;
-
                 const int b = ait % NBUF;
                 { PROF_T0();
                 ok = wait_bounded(tfull_bar(b), (ait / NBUF) & 1u, abort_flag, p.status, DS_TIMEOUT_TMEM_FULL);
@@ -754,18 +738,26 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 // the MMAs of this K block are done: its operands' stage may be refilled
-                if constexpr (PROMO_RELEASE)
-                    if (pw == 0 && lane == 0) ptx::mbar_arrive(empty_bar(ait % STAGES));
+                if constexpr (PROMO_RELEASE) {
+                    if (pw == 0 && lane == 0) ptx::mbar_arrive(empty_bar(stage));
+                    stage = (stage + 1 == STAGES) ? 0 : stage + 1;
+                }
                 if (pw == 0 && lane == 0) PROF_TRACE(4, ait);
                 if (pw == 1 && lane == 0) PROF_TRACE(7, ait);
                 PROF_T0();
                 ptx::tc_fence_after_sync();
                 const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
                                        static_cast<uint32_t>(b * BN + grp * Cfg::COLS);
+                // scale products of this row, one per 64 columns; in flight together with the first TMEM load
+                float sc[Cfg::QUADS];
+                {
+                    const uint32_t sa = slot_addr + (ait % Cfg::SSLOTS) * (Cfg::SSLOT_FLOATS * 4);
+                    if constexpr (Cfg::QUADS == 2) ptx::ld_shared_v2(sa, sc[0], sc[1]);
+                    else ptx::ld_shared_f32(sa, sc[0]);
+                }
                 // partial sums -> registers, 64 columns per load.  Each load and its wait are one asm statement:
                 // the destination registers of a tcgen05.ld are written asynchronously, and code the compiler
                 // places between a load and its wait (a spill, a move) would read them too early.
-                const unsigned long long s_lo2 = pack_f32x2(s_lo, s_lo), s_hi2 = pack_f32x2(s_hi, s_hi);
                 uint32_t v[64];
 #pragma unroll
                 for (int q = 0; q < Cfg::COLS / 64; ++q) {
@@ -780,24 +772,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                             else ptx::mbar_arrive(tempty_bar(b));
                         }
                     }
-                    ptx::fma32_from64<0>(acc[2 * q], v, (2 * q >= hi_from) ? s_hi2 : s_lo2);
-                    ptx::fma32_from64<32>(acc[2 * q + 1], v, (2 * q + 1 >= hi_from) ? s_hi2 : s_lo2);
+                    const unsigned long long s2 = pack_f32x2(sc[q], sc[q]);
+                    ptx::fma32_from64<0>(acc[2 * q], v, s2);
+                    ptx::fma32_from64<32>(acc[2 * q + 1], v, s2);
                 }
-                // Release the a_scale ring entry after its last K block, and only after the FMAs that consumed the
-                // value.  An arrive placed straight after the shared-memory read of a_scale (its value not yet
-                // used) let the producer refill the entry before a slow warp's read had completed: rare 32-row
-                // blocks scaled with the a_scale of a later work unit.
                 if (pw == 0 && lane == 0) PROF_TRACE(5, ait);
                 if (pw == 1 && lane == 0) PROF_TRACE(8, ait);
-                const bool entry_done = (kr == Cfg::SGRP - 1) || (kb == kb1 - 1);
-                if (entry_done) {
-                    __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive(sempty_bar(si));
-                    ++sgit;
-                }
                 PROF_ADD(t_fma);
             }
-            if (u + unit_step < units) fetch_bscale(u + unit_step);      // in flight during the epilogue below
 #ifdef FP8BS_PROFILE
             const long long epi_start = clock64();
             if (pw == 0 && lane == 0) PROF_TRACE(9, static_cast<uint32_t>((u - unit0) / unit_step));
@@ -985,7 +967,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         }
 #ifdef FP8BS_PROFILE
         t_epi += 0;
-        if (pw == 0 && lane == 0) { PROF_OUT(4, w_sfull); PROF_OUT(5, w_tfull); PROF_OUT(6, t_fma); PROF_OUT(7, t_epi); PROF_STAMP(13); }
+        if (pw == 0 && lane == 0) { PROF_OUT(5, w_tfull); PROF_OUT(6, t_fma); PROF_OUT(7, t_epi); PROF_STAMP(13); }
 #endif
         // C must have been read out of shared memory before the CTA goes away
         if (ptx::elect_one()) ptx::tma_store_wait_read<0>();

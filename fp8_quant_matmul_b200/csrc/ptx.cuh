@@ -293,6 +293,16 @@ __device__ __forceinline__ void fma32_from64(unsigned long long (&acc)[16], cons
         : "r"(cur[OFF + 0]), "r"(cur[OFF + 1]), "r"(cur[OFF + 2]), "r"(cur[OFF + 3]), "r"(cur[OFF + 4]), "r"(cur[OFF + 5]), "r"(cur[OFF + 6]), "r"(cur[OFF + 7]), "r"(cur[OFF + 8]), "r"(cur[OFF + 9]), "r"(cur[OFF + 10]), "r"(cur[OFF + 11]), "r"(cur[OFF + 12]), "r"(cur[OFF + 13]), "r"(cur[OFF + 14]), "r"(cur[OFF + 15]), "r"(cur[OFF + 16]), "r"(cur[OFF + 17]), "r"(cur[OFF + 18]), "r"(cur[OFF + 19]), "r"(cur[OFF + 20]), "r"(cur[OFF + 21]), "r"(cur[OFF + 22]), "r"(cur[OFF + 23]), "r"(cur[OFF + 24]), "r"(cur[OFF + 25]), "r"(cur[OFF + 26]), "r"(cur[OFF + 27]), "r"(cur[OFF + 28]), "r"(cur[OFF + 29]), "r"(cur[OFF + 30]), "r"(cur[OFF + 31]), "l"(sc2));
 }
 
+// Shared-memory reads at a 32-bit shared address, kept in program order with the tcgen05 and mbarrier statements.
+__device__ __forceinline__ void ld_shared_v2(uint32_t addr, float& x, float& y)
+{
+    asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x), "=f"(y) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ld_shared_f32(uint32_t addr, float& x)
+{
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(addr) : "memory");
+}
+
 // 64 columns from TMEM, complete on return (load and wait in one statement).
 __device__ __forceinline__ void tmem_ld_x64_sync(uint32_t taddr, uint32_t (&v)[64])
 {

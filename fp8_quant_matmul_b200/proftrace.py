@@ -17,7 +17,7 @@ from . import api
 
 PROF_LIB = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libfp8bs_prof.so")
 COUNTERS = ["producer wait: free stage", "MMA wait: free TMEM buffer", "MMA wait: operands", "MMA loop total",
-            "promotion wait: a_scale", "promotion wait: partial sums", "promotion loads + FMAs", "epilogue"]
+            "(not used)", "promotion wait: partial sums", "promotion loads + FMAs", "epilogue"]
 STAMPS = ["start", "set-up done", "first operands (lead CTA)", "MMA loop done", "promotion loop done", "all stores issued",
           "exit"]
 
@@ -59,13 +59,13 @@ def trace(M, N, K, path=0, splits=0, tile_n=0, kblocks=40):
             print("   t[%-26s] min %8d ns   mean %8.0f   max %8d" % (name, col.min() - t0, col.mean() - t0, col.max() - t0))
     z = tr[1, 0]
     KB = K // 128
-    print("   kb : stage free | TMEM free  operands  MMAs issued | a_scale  partial sums  FMAs done | warp 5: partial sums  FMAs done"
+    print("   kb : stage free | TMEM free  operands  MMAs issued | partial sums  FMAs done | warp 5: partial sums  FMAs done"
           "   (clock cycles of CTA 0, relative to its first operands)")
     for i in range(min(128, kblocks)):
         if tr[2, i] == 0:
             break
-        r = [int(tr[e, i] - z) if tr[e, i] else 0 for e in (6, 0, 1, 2, 3, 4, 5, 7, 8)]
-        print("   %3d: %9d | %9d %9d %9d | %9d %9d %9d | %9d %9d" % ((i,) + tuple(r)))
+        r = [int(tr[e, i] - z) if tr[e, i] else 0 for e in (6, 0, 1, 2, 4, 5, 7, 8)]
+        print("   %3d: %9d | %9d %9d %9d | %9d %9d | %9d %9d" % ((i,) + tuple(r)))
     units = [(int(tr[9, i] - z), int(tr[10, i] - z)) for i in range(128) if tr[9, i]]
     if units and KB <= 16:
         print("   epilogue of CTA 0's units (start, end): " + " ".join("(%d, %d)" % u for u in units[:16]))
