@@ -39,10 +39,14 @@
 //              128-byte swizzled: the MN-major operand layout tcgen05.mma reads directly.  The
 //              byte-wise transposing copy of the reference (mn_large.hip:40-48) has no
 //              counterpart here.
-//   warp 1     MMA issuer.  Per 128-K block: four tcgen05.mma kind::f8f6f4 (K = 32 each) into a
-//              fresh TMEM buffer (the first one overwrites), then a commit that publishes the TMEM
-//              buffer and, in the three-stage kernels, a second one that frees the shared-memory stage
-//              (with four or more stages a promotion warp frees it, see PROMO_RELEASE).
+//   warp 1     MMA issuer.  Per 128-K block and 128-column part of the tile: four tcgen05.mma kind::f8f6f4 (K = 32
+//              each) into a fresh TMEM buffer (the first one overwrites) and a commit that publishes the part; after
+//              the last part a commit that frees the shared-memory stage.  The two parts of a 256-wide tile have
+//              barriers of their own and belong to different promotion warps, so the MMAs of one part run while
+//              the other is handed over and back.  With whole K blocks the chain MMA 512 + commit + promotion +
+//              hand-back of a TMEM buffer (1580 cycles, two buffers) set a period of 790 cycles per K block; with
+//              parts it is 735 (instrumented), and loads and power set it.  Measured: 6144 x 4608 x 7168 164-169
+//              -> 158 us, 1024 x 3072 x 1536 10.2 -> 9.5, 6144 x 4096 x 512 20.2 -> 19.4.
 //   (Each of these roles is one thread, chosen by elect.sync, see ptx::elect_one.)
 //   warp 2     scale products: a_scale * b_scale of the tile's rows and 64-column pieces into shared memory, one slot
 //              per K block (the reference stages the pre-multiplied scales in LDS too, mn_large.hip:50-55).  The promotion
@@ -118,6 +122,7 @@ struct TileCfg {
     static constexpr int STAGE_BYTES = SLAB * (1 + NBOX_B);
     static constexpr int TMEM_COLS = 512;
     static constexpr int NBUF = TMEM_COLS / BN;       // TMEM partial-sum buffers
+    static constexpr int NH = BN / 128;               // 128-column parts of a tile that are handed over separately
     static constexpr int COLS = BN / 2;               // columns of the tile row a promotion thread owns (64 or 128)
     static constexpr int NCH = COLS / 32;             // ... as 32-column chunks
     static constexpr int PROMO_WARPS = 8;             // 4 TMEM lane quarters x 2 column groups
@@ -136,7 +141,7 @@ struct TileCfg {
     static constexpr int FIXED = 1024 + STG_BYTES + SRING_BYTES + 512;
     static constexpr int STAGES = (SMEM_LIMIT - FIXED) / STAGE_BYTES;
     static_assert(STAGES >= 2, "pipeline depth");
-    static constexpr int NUM_BARS = 2 * STAGES + 2 * NBUF;
+    static constexpr int NUM_BARS = 2 * STAGES + 2 * NBUF * NH;
     static_assert(NUM_BARS * 8 + 64 <= 512, "barrier area");
     static constexpr int SMEM_BYTES = FIXED + STAGES * STAGE_BYTES;
 };
@@ -279,7 +284,7 @@ __device__ __forceinline__ void stage_and_store_64(const CUtensorMap* tmC, int n
 // caller has made sure that both boxes are free (wait_read<0> in that thread).
 template <class Cols0, class Cols1>
 __device__ __forceinline__ void stage_and_store_2x64(const CUtensorMap* tmC, int n_dest, uint8_t* stg, uint32_t stg_addr,
-                                                     int lane, const Cols0 c0, const Cols1 c1, int col, int row0, int M, int N)
+                                                     int lane, const Cols0 c0, const Cols1 c1, int col, int col1, int row0, int M, int N)
 {
     stage_64(stg, lane, c0);
     stage_64(stg + 4096, lane, c1);
@@ -288,7 +293,7 @@ __device__ __forceinline__ void stage_and_store_2x64(const CUtensorMap* tmC, int
     if (col < N && row0 < M && ptx::elect_one()) {
         for (int d = 0; d < n_dest; ++d) {
             ptx::tma_store_2d(tmC + d, stg_addr, col, row0);
-            if (col + 64 < N) ptx::tma_store_2d(tmC + d, stg_addr + 4096, col + 64, row0);
+            if (col1 < N) ptx::tma_store_2d(tmC + d, stg_addr + 4096, col1, row0);
         }
         ptx::tma_store_commit();
     }
@@ -320,17 +325,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     using Cfg = TileCfg<BN, CG>;
     constexpr int STAGES = Cfg::STAGES;
     constexpr int NBUF = Cfg::NBUF;
+    constexpr int NH = Cfg::NH;
     constexpr bool SPLITK = (MODE == 1 || MODE == 2);   // K cut into p.splits equal ranges per tile
     constexpr bool STREAMK = (MODE == 3);               // K blocks of all tiles dealt out evenly, see below
     static_assert(MODE != 2 || CG == 1, "the cluster reduction uses the cluster for the K splits");
     static_assert(MODE != 3 || CG == 1, "stream-K is built for single-CTA tiles");
     constexpr bool RESIDENT = (MODE == 4);              // both K blocks of a tile kept in TMEM (K <= 256)
-    // Who frees a shared-memory stage.  Every tcgen05 instruction costs the issuing thread time, so with four or more
-    // stages the MMA warp issues one commit per K block (TMEM buffer full) and a promotion warp, which learns from that
-    // barrier that the MMAs are done, arrives on the stage's barrier: 1.5-4 % faster on the pair and the 128-wide
-    // kernels.  With three stages (256-wide single-CTA tiles) the later release starves the loads (3-7 % slower),
-    // so there the MMA warp frees the stage with a second commit.
-    constexpr bool PROMO_RELEASE = (STAGES >= 4) && !RESIDENT;
     static_assert(!RESIDENT || (CG == 1 && BN == 256), "the short-K mode uses 256-wide single-CTA tiles");
     // MODE 2: fp32 partial tile of this CTA, rows padded by 16 bytes so that a warp's 32 rows hit distinct banks
     constexpr int PART_PITCH = BN * 4 + 16;
@@ -351,8 +351,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     // ctrl[0] TMEM base address, ctrl[1] abort flag, ctrl[2] "this CTA reduces the tile"
     auto full_bar = [&](int s) { return bar_base + 8u * s; };
     auto empty_bar = [&](int s) { return bar_base + 8u * (STAGES + s); };
-    auto tfull_bar = [&](int b) { return bar_base + 8u * (2 * STAGES + b); };
-    auto tempty_bar = [&](int b) { return bar_base + 8u * (2 * STAGES + NBUF + b); };
+    auto tfull_bar = [&](int h, int b) { return bar_base + 8u * (2 * STAGES + h * NBUF + b); };
+    auto tempty_bar = [&](int h, int b) { return bar_base + 8u * (2 * STAGES + (NH + h) * NBUF + b); };
 
     const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);   // uniform, and known to be
     const int lane = threadIdx.x & 31;
@@ -370,10 +370,11 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             ptx::mbar_init(full_bar(s), 1);
             ptx::mbar_init(empty_bar(s), 1);
         }
-        for (int b = 0; b < NBUF; ++b) {
-            ptx::mbar_init(tfull_bar(b), 2);                         // the MMA warp's commit and the scale warp
-            ptx::mbar_init(tempty_bar(b), Cfg::PROMO_WARPS * CG);   // the leader also hears from the peer's warps
-        }
+        for (int h = 0; h < NH; ++h)
+            for (int b = 0; b < NBUF; ++b) {
+                ptx::mbar_init(tfull_bar(h, b), 2);                                // the MMA warp's commit and the scale warp
+                ptx::mbar_init(tempty_bar(h, b), Cfg::PROMO_WARPS / NH * CG);      // the leader also hears from the peer's warps
+            }
         ctrl[1] = 0u;
         ctrl[2] = 0u;
         ptx::fence_mbar_init();
@@ -445,6 +446,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         n0 = ni * BN;
     };
 
+    // First column, within the tile, of the 64-column piece q of column group g.  A pair's MMA of part h takes 64 columns
+    // from each CTA's B slab (slab r holds the tile's columns 128 r ..), which come out as the part's two pieces.
+    auto col_of = [](int g, int q) { return CG == 2 ? g * 64 + q * 128 : g * Cfg::COLS + q * 64; };
+
     if (warp < 4) {
         ptx::setmaxnreg_dec<64>();
         if (warp == 0 && ptx::elect_one()) {
@@ -494,7 +499,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             }
         } else if (warp == 1 && rank == 0 && ptx::elect_one()) {
             // ---------------------------------------------------- MMA issuer ----------------
-            constexpr uint32_t idesc = ptx::make_idesc_e4m3_mnmajor(Cfg::TILE_M, BN);
+            constexpr uint32_t idesc = ptx::make_idesc_e4m3_mnmajor(Cfg::TILE_M, BN / NH);
+            // B descriptor of part h: its own slab, or with a pair 64 columns of each CTA's slab (see col_of)
+            constexpr uint64_t BSTEP = (CG == 2 ? 64 : Cfg::SLAB) >> 4;
             uint32_t it = 0, ait = 0, tcount = 0, sphase = 0;
             int stage = 0;
             bool ok = true;
@@ -505,15 +512,45 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             for (int u = unit0; u < units && ok; u += unit_step) {
                 int tile, m0, n0, kb0, kb1;
                 decode(u, tile, m0, n0, kb0, kb1);
+                if constexpr (RESIDENT) {
+                    // MODE 4: K block j of a tile goes to buffer j; part h of the tile, with all its K blocks, is handed over
+                    // once and taken back once per tile (barriers number 0, phase = tile count)
+                    for (int h = 0; h < NH && ok; ++h) {
+                        int st = stage;
+                        uint32_t sph = sphase;
+                        for (int kb = kb0; kb < kb1; ++kb) {
+                            if (h == 0) {
+                                ok = wait_bounded(full_bar(st), sph, abort_flag, p.status, DS_TIMEOUT_STAGE_FULL);
+                                if (!ok) break;
+                            }
+                            if (kb == kb0) {
+                                ok = wait_bounded(tempty_bar(h, 0), (tcount & 1u) ^ 1u, abort_flag, p.status, DS_TIMEOUT_TMEM_EMPTY);
+                                if (!ok) break;
+                            }
+                            ptx::tc_fence_after_sync();
+                            const uint32_t a_addr = stage_base + st * Cfg::STAGE_BYTES;
+                            const uint64_t adesc = ptx::make_smem_desc_sw128(a_addr, Cfg::SLAB, 1024);
+                            const uint64_t bdesc = ptx::make_smem_desc_sw128(a_addr + Cfg::SLAB, Cfg::SLAB, 1024) + h * BSTEP;
+                            const uint32_t d = tmem_base + static_cast<uint32_t>((kb - kb0) * BN + h * (BN / NH));
+#pragma unroll
+                            for (int j = 0; j < 4; ++j) {
+                                const uint64_t step = static_cast<uint64_t>(j * (4096 >> 4));
+                                ptx::mma_f8f6f4(d, adesc + step, bdesc + step, idesc, j > 0 ? 1u : 0u);
+                            }
+                            if (h == NH - 1) ptx::mma_commit(empty_bar(st));
+                            if (++st == STAGES) { st = 0; sph ^= 1u; }
+                        }
+                        if (!ok) break;
+                        ptx::mma_commit(tfull_bar(h, 0));
+                        if (h == NH - 1) { stage = st; sphase = sph; }
+                    }
+                } else
                 for (int kb = kb0; kb < kb1; ++kb, ++it, ++ait) {
                     const int s = stage;
                     const uint32_t ph = sphase;
                     if (++stage == STAGES) { stage = 0; sphase ^= 1u; }
-                    // MODE 4: K block j of a tile goes to buffer j; the pair is handed over and taken back once per tile
-                    // (barriers tfull / tempty number 0, phase = tile count)
-                    const int b = RESIDENT ? (kb - kb0) : static_cast<int>(ait % NBUF);
-                    const uint32_t bph = RESIDENT ? (tcount & 1u) : ((ait / NBUF) & 1u);
-                    const int eb = RESIDENT ? 0 : b;                       // the barrier pair that guards this buffer
+                    const int b = ait % NBUF;
+                    const uint32_t bph = (ait / NBUF) & 1u;
                     // operands first (they are usually there already), then the TMEM buffer: nothing but the MMA
                     // issue stands between the promotion warps' release of the buffer and its reuse
                     { PROF_T0();
@@ -521,38 +558,36 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                     PROF_ADD(w_full); }
                     if (!ok) break;
                     PROF_TRACE(1, it);
-                    if (!RESIDENT || kb == kb0) {
-                        PROF_T0();
-                        ok = wait_bounded(tempty_bar(eb), bph ^ 1u, abort_flag, p.status, DS_TIMEOUT_TMEM_EMPTY);
-                        PROF_ADD(w_tempty);
-                    }
-                    if (!ok) break;
-                    PROF_TRACE(0, it);
-#ifdef FP8BS_PROFILE
-                    if (it == 0) { PROF_STAMP(10); }
-#endif
-                    ptx::tc_fence_after_sync();
                     const uint32_t a_addr = stage_base + s * Cfg::STAGE_BYTES;
                     const uint64_t adesc = ptx::make_smem_desc_sw128(a_addr, Cfg::SLAB, 1024);
-                    const uint64_t bdesc = ptx::make_smem_desc_sw128(a_addr + Cfg::SLAB, Cfg::SLAB, 1024);
-                    const uint32_t d = tmem_base + static_cast<uint32_t>(b * BN);
+                    const uint64_t bdesc0 = ptx::make_smem_desc_sw128(a_addr + Cfg::SLAB, Cfg::SLAB, 1024);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        // K = 32 per instruction = 4 swizzle atoms of 8 k-rows = 4096 bytes
-                        const uint64_t step = static_cast<uint64_t>(j * (4096 >> 4));
-                        if constexpr (CG == 2) ptx::mma_f8f6f4_pair(d, adesc + step, bdesc + step, idesc, j > 0 ? 1u : 0u);
-                        else ptx::mma_f8f6f4(d, adesc + step, bdesc + step, idesc, j > 0 ? 1u : 0u);
+                    for (int h = 0; h < NH; ++h) {
+                        { PROF_T0();
+                        ok = wait_bounded(tempty_bar(h, b), bph ^ 1u, abort_flag, p.status, DS_TIMEOUT_TMEM_EMPTY);
+                        PROF_ADD(w_tempty); }
+                        if (!ok) break;
+                        if (h == 0) PROF_TRACE(0, it);
+#ifdef FP8BS_PROFILE
+                        if (it == 0 && h == 0) { PROF_STAMP(10); }
+#endif
+                        ptx::tc_fence_after_sync();
+                        const uint64_t bdesc = bdesc0 + h * BSTEP;
+                        const uint32_t d = tmem_base + static_cast<uint32_t>(b * BN + h * (BN / NH));
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            // K = 32 per instruction = 4 swizzle atoms of 8 k-rows = 4096 bytes
+                            const uint64_t step = static_cast<uint64_t>(j * (4096 >> 4));
+                            if constexpr (CG == 2) ptx::mma_f8f6f4_pair(d, adesc + step, bdesc + step, idesc, j > 0 ? 1u : 0u);
+                            else ptx::mma_f8f6f4(d, adesc + step, bdesc + step, idesc, j > 0 ? 1u : 0u);
+                        }
+                        // with a pair, one commit reaches both CTAs
+                        if constexpr (CG == 2) ptx::mma_commit_pair_all(tfull_bar(h, b), 3);
+                        else ptx::mma_commit(tfull_bar(h, b));
                     }
-                    // the promotion warps wait on this one; the producer is several stages ahead
-                    if constexpr (CG == 2) {
-                        // one commit per barrier reaches both CTAs of the pair (with plain commits, two per barrier, the
-                        // fourth one of a K block cost ~100 cycles of tensor-pipe time)
-                        ptx::mma_commit_pair_all(tfull_bar(b), 3);
-                        if constexpr (!PROMO_RELEASE) ptx::mma_commit_pair_all(empty_bar(s), 3);
-                    } else {
-                        if (!RESIDENT || kb == kb1 - 1) ptx::mma_commit(tfull_bar(eb));
-                        if constexpr (!PROMO_RELEASE) ptx::mma_commit(empty_bar(s));
-                    }
+                    if (!ok) break;
+                    if constexpr (CG == 2) ptx::mma_commit_pair_all(empty_bar(s), 3);
+                    else ptx::mma_commit(empty_bar(s));
                     PROF_TRACE(2, it);
                 }
                 ++tcount;
@@ -609,7 +644,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                     if (!ok) break;
                     if (!valid[d]) { ok = false; break; }       // no more K blocks
                     if ((!RESIDENT || kpos == 0) && item >= NB) {
-                        ok = wait_bounded(tfull_bar(item % NB), ((item / NB) - 1u) & 1u, abort_flag, p.status, DS_TIMEOUT_SCALE_EMPTY);
+#pragma unroll
+                        for (int h = 0; h < NH && ok; ++h)
+                            ok = wait_bounded(tfull_bar(h, item % NB), ((item / NB) - 1u) & 1u, abort_flag, p.status, DS_TIMEOUT_SCALE_EMPTY);
                         ok = __all_sync(0xffffffffu, ok);
                         if (!ok) break;
                     }
@@ -624,12 +661,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                         for (int g = 0; g < 2; ++g) {
                             float* w = dst + (g * 128 + 32 * j) * Cfg::QUADS;
                             if constexpr (Cfg::QUADS == 2)
-                                *reinterpret_cast<float2*>(w) = make_float2(av[d][j] * bs[2 * g], av[d][j] * bs[2 * g + 1]);
+                                *reinterpret_cast<float2*>(w) = make_float2(av[d][j] * bs[col_of(g, 0) / 64], av[d][j] * bs[col_of(g, 1) / 64]);
                             else *w = av[d][j] * bs[g];
                         }
                     if (!RESIDENT || kpos == KB - 1) {
                         __syncwarp();
-                        if (lane == 0) ptx::mbar_arrive(tfull_bar(RESIDENT ? 0 : item % NB));
+                        if (lane < NH) ptx::mbar_arrive(tfull_bar(lane, RESIDENT ? 0 : item % NB));
                         ++item;
                         kpos = 0;
                     } else {
@@ -646,21 +683,22 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         const int pw = warp - 4;
         const int quarter = warp & 3;            // TMEM lanes this warp may read: 32*quarter ..
         const int grp = pw >> 2;                 // which half of the tile's columns
+        const int part = (NH == 2) ? grp : 0;    // ... and which of the tile's separately handed-over parts they are in
         const int row_in_tile = quarter * 32 + lane;
         uint8_t* my_stg = stg_ptr + pw * 4096 * Cfg::NSTG;
         const uint32_t my_stg_addr = stg_base + pw * 4096 * Cfg::NSTG;
-        uint32_t lead_tempty = tempty_bar(0);
-        if constexpr (CG == 2) lead_tempty = ptx::mapa(tempty_bar(0), 0);
+        uint32_t lead_tempty = tempty_bar(part, 0);
+        if constexpr (CG == 2) lead_tempty = ptx::mapa(tempty_bar(part, 0), 0);
         const uint32_t slot_addr = sring_base + static_cast<uint32_t>((grp * 128 + row_in_tile) * Cfg::QUADS * 4);
         uint32_t ait = 0;
-        uint32_t stage = 0;                      // ait % STAGES
         uint32_t tcount = 0;                     // MODE 4: tiles done by this CTA
         bool ok = true;
         PROF_DECL(w_tfull); PROF_DECL(t_fma); PROF_DECL(t_epi);
         for (int u = unit0; u < units; u += unit_step) {
             int tile, m0, n0, kb0, kb1;
             decode(u, tile, m0, n0, kb0, kb1);
-            const int ncol0 = n0 + grp * Cfg::COLS;           // first local column of this thread
+            const int ncol0 = n0 + col_of(grp, 0);            // first local columns of this thread's pieces
+            const int ncol1 = n0 + col_of(grp, 1);
             // running sums of this thread's row: 4 chunks of 32 columns, two fp32 per 64-bit register
             unsigned long long acc[Cfg::NCH][16];
 #pragma unroll
@@ -673,7 +711,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 const bool two = (kb1 - kb0) > 1;
                 // the previous stores have read both boxes before anything is staged into them
                 if (ptx::elect_one()) ptx::tma_store_wait_read<0>();
-                ok = wait_bounded(tfull_bar(0), tcount & 1u, abort_flag, p.status, DS_TIMEOUT_TMEM_FULL);
+                ok = wait_bounded(tfull_bar(part, 0), tcount & 1u, abort_flag, p.status, DS_TIMEOUT_TMEM_FULL);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 ptx::tc_fence_after_sync();
@@ -695,7 +733,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                         // the whole tile is in registers or staged: the MMA warp may fill TMEM for the next tile
                         ptx::tc_fence_before_sync();
                         __syncwarp();
-                        if (lane == 0) ptx::mbar_arrive(tempty_bar(0));
+                        if (lane == 0) ptx::mbar_arrive(tempty_bar(part, 0));
                     }
 #pragma unroll
                     for (int i = 0; i < 16; ++i) { acc[0][i] = 0ull; acc[1][i] = 0ull; }
@@ -733,15 +771,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             for (int kb = kb0; kb < kb1 && ok; ++kb, ++ait) {
                 const int b = ait % NBUF;
                 { PROF_T0();
-                ok = wait_bounded(tfull_bar(b), (ait / NBUF) & 1u, abort_flag, p.status, DS_TIMEOUT_TMEM_FULL);
+                ok = wait_bounded(tfull_bar(part, b), (ait / NBUF) & 1u, abort_flag, p.status, DS_TIMEOUT_TMEM_FULL);
                 PROF_ADD(w_tfull); }
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
-                // the MMAs of this K block are done: its operands' stage may be refilled
-                if constexpr (PROMO_RELEASE) {
-                    if (pw == 0 && lane == 0) ptx::mbar_arrive(empty_bar(stage));
-                    stage = (stage + 1 == STAGES) ? 0 : stage + 1;
-                }
                 if (pw == 0 && lane == 0) PROF_TRACE(4, ait);
                 if (pw == 1 && lane == 0) PROF_TRACE(7, ait);
                 PROF_T0();
@@ -769,7 +802,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                         __syncwarp();
                         if (lane == 0) {
                             if constexpr (CG == 2) ptx::mbar_arrive_cluster(lead_tempty + 8u * b);
-                            else ptx::mbar_arrive(tempty_bar(b));
+                            else ptx::mbar_arrive(tempty_bar(part, b));
                         }
                     }
                     const unsigned long long s2 = pack_f32x2(sc[q], sc[q]);
@@ -794,13 +827,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                     __syncwarp();
                     if (u + unit_step < units) {
                         stage_and_store_2x64(cmaps.m, p.n_dest, my_stg, my_stg_addr, lane, PackedCols{acc[0], acc[1]},
-                                             PackedCols{acc[2], acc[3]}, ncol0, m0 + quarter * 32, p.M, p.N);
+                                             PackedCols{acc[2], acc[3]}, ncol0, ncol1, m0 + quarter * 32, p.M, p.N);
                     } else {
                         // the CTA's last tile: the first store leaves while the second box is being staged (shorter tail)
                         stage_and_store_64<-1>(cmaps.m, p.n_dest, my_stg, my_stg_addr, lane, PackedCols{acc[0], acc[1]},
                                                ncol0, m0 + quarter * 32, p.M, p.N);
                         stage_and_store_64<-1>(cmaps.m, p.n_dest, my_stg + 4096, my_stg_addr + 4096, lane,
-                                               PackedCols{acc[2], acc[3]}, ncol0 + 64, m0 + quarter * 32, p.M, p.N);
+                                               PackedCols{acc[2], acc[3]}, ncol1, m0 + quarter * 32, p.M, p.N);
                     }
                 } else {
                     stage_and_store_64<0>(cmaps.m, p.n_dest, my_stg, my_stg_addr, lane, PackedCols{acc[0], acc[1]}, ncol0,
@@ -887,8 +920,12 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 }
             } else if constexpr (MODE == 2) {
                 // ---- split-K through the cluster: leave this K range's partial tile in shared memory ----
-                // The stage buffers are free: every MMA of this CTA has completed (the last TMEM buffer was full)
-                // and every load that was issued has been consumed.
+                // The stage buffers are free once every MMA of this CTA has completed: the last part of the last K block is
+                // full (with two parts, the other warps' one may still be computed from the operands in them).
+                if (NH == 2 && ok) {
+                    ok = wait_bounded(tfull_bar(NH - 1, (ait - 1) % NBUF), ((ait - 1) / NBUF) & 1u, abort_flag, p.status, DS_TIMEOUT_TMEM_FULL);
+                    ok = __all_sync(0xffffffffu, ok);
+                }
                 if (ok) {
                     float4* dst = reinterpret_cast<float4*>(aligned + row_in_tile * PART_PITCH + grp * Cfg::COLS * 4);
 #pragma unroll
@@ -956,7 +993,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                                 sum[4 * j + 3] += v.w;
                             }
                         }
-                        stage_and_store_64<0>(cmaps.m, p.n_dest, my_stg, my_stg_addr, lane, FloatCols{sum}, ncol0 + h * 64, m0 + quarter * 32, p.M, p.N);
+                        stage_and_store_64<0>(cmaps.m, p.n_dest, my_stg, my_stg_addr, lane, FloatCols{sum}, h ? ncol1 : ncol0, m0 + quarter * 32, p.M, p.N);
                     }
                 }
             }
