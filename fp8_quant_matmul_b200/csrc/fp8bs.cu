@@ -411,6 +411,19 @@ static int encode_c_map(CUtensorMap* tm, void* base, int M, int N, int ld)
     return FP8BS_OK;
 }
 
+// Tile order: groups of this many row blocks (256 rows each with a pair, else 128), column by column within a group.  The
+// tiles in flight at one time are then about as many rows as columns, so that they share operands: walking all rows first
+// reads all of A anew for every few columns, which no longer comes from L2 once A is larger than that.  Measured in groups of
+// 4, 6, 8, 12, 16 and all row blocks: 16384 x 4608 x 7168 (A is 117 MB) 409 / 410 / 413 / 414 / 415 / 494 us, 16384 x 576 x
+// 7168 76 / 76 / 76 / 78 / 78 / 84, 8192 x 4608 x 7168 207 / 208 / 209 / 209 / 209 / 215; with 4096 or 6144 rows and K <= 2304
+// the groups gain nothing and cost up to 1.5 % (4096 x 7168 x 2048, 6144 x 7168 x 2304), hence the lower bound on A.
+constexpr long long GROUPED_A_BYTES = 32ll << 20;
+static int tile_group(int m_tiles, int cg, long long a_bytes)
+{
+    const int g = cg == 2 ? 6 : 12;
+    return (m_tiles > g && a_bytes >= GROUPED_A_BYTES) ? g : m_tiles;
+}
+
 struct TensorMaps {
     CUtensorMap A, B;
     CMaps C;
@@ -523,7 +536,11 @@ static int gemm_impl(const void* A, const void* B, const float* a_scale, const f
     p.sn = ceil_div(n_total, 128);
     p.m_tiles = ceil_div(M, 128 * cfg.cg);
     p.n_tiles = ceil_div(N, cfg.tile_n);
-    p.inv_m_tiles = 1.0f / static_cast<float>(p.m_tiles);
+    p.group = tile_group(p.m_tiles, cfg.cg, static_cast<long long>(M) * K);
+    p.group_tiles = p.group * p.n_tiles;
+    p.inv_group_tiles = 1.0f / static_cast<float>(p.group_tiles);
+    p.inv_group = 1.0f / static_cast<float>(p.group);
+    p.inv_last_group = (p.m_tiles % p.group) ? 1.0f / static_cast<float>(p.m_tiles % p.group) : p.inv_group;
     p.splits = cfg.splits;
     p.n_dest = dests ? n_dest : 1;
     p.elem_scale = 1.0f;

@@ -101,7 +101,10 @@ struct GemmParams {
     int n_off;               // global column index of local column 0 (N-sharded calls), else 0
     int sn;                  // rows of b_scale = ceil(N_total / 128)  (check.cu:36)
     int m_tiles, n_tiles, splits;
-    float inv_m_tiles;       // 1 / m_tiles, for the tile -> (row block, column block) decode
+    int group;               // tile order: groups of this many row blocks, see decode
+    int group_tiles;         // group * n_tiles
+    float inv_group_tiles;   // their reciprocals, and that of the last (shorter) group's height
+    float inv_group, inv_last_group;
     int n_dest;              // number of valid entries of the CMaps argument (1 = only the caller's C)
     float elem_scale;        // folded into b_scale: 1 for e4m3fn bytes
 #ifdef FP8BS_PROFILE
@@ -423,8 +426,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     const int unit0 = STREAMK ? 0 : group_id;          // a CTA's (pair's) first work unit and its stride
     const int unit_step = STREAMK ? 1 : num_groups;
 
-    // unit -> (tile, split) -> (row of this CTA, first column, K-block range).  Tiles are numbered
-    // m-fastest so CTAs that run side by side share the B slab through L2.
+    // unit -> (tile, split) -> (row of this CTA, first column, K-block range).
     auto decode = [&](int u, int& tile, int& m0, int& n0, int& kb0, int& kb1) {
         if constexpr (STREAMK) {
             tile = sk_first + u;
@@ -436,12 +438,20 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             kb0 = SPLITK ? (split * KB) / p.splits : 0;
             kb1 = SPLITK ? ((split + 1) * KB) / p.splits : KB;
         }
-        // tile = ni * m_tiles + mi without an integer division (some 100 cycles, twice per tile in every role): the
-        // float quotient is off by at most one for tile counts below 2^22, and the remainder says which way
-        int ni = __float2int_rz(__int2float_rn(tile) * p.inv_m_tiles);
-        int mi = tile - ni * p.m_tiles;
-        if (mi < 0) { --ni; mi += p.m_tiles; }
-        else if (mi >= p.m_tiles) { ++ni; mi -= p.m_tiles; }
+        // Tiles are numbered in groups of p.group row blocks, column by column within a group and m-fastest within a
+        // column.  Quotients by float reciprocal instead of integer division (some 100 cycles each, in every role and
+        // tile): off by at most one for tile counts below 2^22, and the remainder says which way.
+        auto divide = [](int x, int d, float inv, int& q, int& r) {
+            q = __float2int_rz(__int2float_rn(x) * inv);
+            r = x - q * d;
+            if (r < 0) { --q; r += d; }
+            else if (r >= d) { ++q; r -= d; }
+        };
+        int gi = 0, rem = tile, ni, mi;
+        if (p.group < p.m_tiles) divide(tile, p.group_tiles, p.inv_group_tiles, gi, rem);
+        const int first = gi * p.group, left = p.m_tiles - first;
+        divide(rem, left < p.group ? left : p.group, left < p.group ? p.inv_last_group : p.inv_group, ni, mi);
+        mi += first;
         m0 = mi * Cfg::TILE_M + static_cast<int>(rank) * Cfg::BM;
         n0 = ni * BN;
     };
