@@ -221,55 +221,56 @@ static int stream_k_ctas(int tiles, int KB, int sm_count)
 }
 
 
-// Estimated run time of a configuration in microseconds.  The constants come from a measured sweep of
-// every configuration over the 18 benchmark shapes on a B200 (power-capped, cold L2):
-//   per 128-K block of one work unit: 0.44 us (128-wide tile), 0.53 us (256-wide), 0.505 us (256 x 256 pair, with
-//   one multicast commit per K block and the stages freed by a promotion warp: the pair wins from K = 1536 on,
-//   2 % at K = 1536 and M = 6144 (equal at M = 1024), 3-5 % from K = 2048 on; at K = 512 it is 2-8 % slower);
-//   per work unit (tile switch, epilogue): 0.35 / 1.2 / 1.40 us;  per launch: 3.5 us;
-//   split-K through a workspace: 3.5 us + 1 us per split and 128 columns for the partial-sum round trip, doubled
-//   when a CTA has to walk more than one unit (the last-arriver reduction then delays the next unit);
+// Estimated run time of a configuration in microseconds.  The constants are a least-squares fit to a sweep of every
+// configuration over 85 shapes on a B200 (the 18 benchmark shapes and random ones, M 80..16384, N 64..7168, K 128..7168, cold
+// L2, launches back to back); choosing by it costs 0.8 % on average against the best configuration of each shape, 16 % at
+// most (the constants before it, fitted to slower kernels, 3.7 %).  The overheads of the two split-K forms are 1.5 and 0.6 us above
+// the fit, which settles near ties for the kernel that does not cut K.  Per 128-K block of a work unit 0.23 us (128-wide tile), 0.45 (256-wide), 0.41 (256 x 256 pair), and up to 27 % / 15 %
+// / 0 % more the more SMs take part; per work unit 1.9 / 1.5 / 1.5 us (tile switch, epilogue), 3 us per launch.
+// Examples, 128-wide / 256-wide / pair: 1024 x 7168 x 2304 23.1 / 22.9 / 20.0 us, 128 x 7168 x 2304 9.2 / 13.3 / 11.8, 1024 x
+// 1536 x 7168 18.7 / 28.0 / 23.9 (best with K cut: 20.7).
+//   split-K through a workspace: 2.15 us + 1.1 us per split and 128 columns for the partial-sum round trip, four times
+//   that when a CTA has to walk more than one unit (the last-arriver reduction then delays the next unit);
 //   split-K inside a cluster: one CTA per (tile, K range); the number of clusters that fit on the GPU at once is
-//   cudaOccupancyMaxActiveClusters for this kernel's footprint (one CTA per SM), tabulated below for a B200;
-//   overhead 2 us (3 us for 256-wide tiles) + 0.5 us per split and 128 columns (shared-memory round trip, two
-//   cluster barriers), paid again with 3 us of prologue by every further wave of clusters.
-// Stream-K hand-over per 128 columns of tile width: a CTA first leaves a partial tile in the workspace (its promotion
-// warps are busy with that while its MMA warp runs dry) and at the end reads its neighbours'; CTAs that run side by side
-// are also on tiles far apart and share less through L2.  Measured 6-11 us in total on the benchmark shapes, which
-// is why the estimate keeps stream-K for shapes with very few, very long tiles only.
-constexpr double STREAM_K_FIXUP_US = 6.0;
+//   cudaOccupancyMaxActiveClusters for this kernel's footprint (one CTA per SM); overhead 2.2 us (5.2 us for 256-wide
+//   tiles), paid again with 4.1 us of prologue by every further wave of clusters;
+//   stream-K: 2.9 us per 128 columns of tile width for the hand-over of partial tiles, times half the number of CTAs that
+//   share a tile (the finishing CTA reads the others' one after the other).
 // Mode 4 (K <= 256, partial sums resident in TMEM) is chosen by rule, see choose_config.
 constexpr int SHORT_K_MAX_WAVES = 3;
 static double config_cost(const DeviceModel& dm, int M, int N, int K, int tile_n, int splits, int cg, int mode)
 {
     const int KB = K / 128;
     const int tiles = ceil_div(M, 128 * cg) * ceil_div(N, tile_n);
+    const int kind = (cg == 2) ? 2 : (tile_n == 256 ? 1 : 0);
+    static const double PER_KB[3] = {0.232, 0.452, 0.407}, CROWDING[3] = {0.274, 0.147, 0.0}, PER_UNIT[3] = {1.875, 1.529, 1.533};
+    constexpr double LAUNCH_US = 3.0;
+    // K block time when `ctas` CTAs are at work
+    auto per_kb = [&](int ctas) { return PER_KB[kind] * (1.0 + CROWDING[kind] * ctas / dm.sm_count); };
     if (mode == 3) {
         // every CTA: ceil(T / G) K blocks, its share of the tile switches, one partial-sum hand-over each way
         const int g = stream_k_ctas(tiles, KB, dm.sm_count);
         const long long total = static_cast<long long>(tiles) * KB;
         const double kb_each = static_cast<double>((total + g - 1) / g);
-        const double per_kb3 = (tile_n == 256 ? 0.53 : 0.44), per_unit3 = (tile_n == 256 ? 1.2 : 0.35);
         // the CTA that finishes a tile reads the partial tile of every other CTA that worked on it, one after the other
         const double sharers = (kb_each < KB) ? (KB / kb_each + 1.0) : 2.0;
-        return 3.5 + kb_each * per_kb3 + (static_cast<double>(tiles) / g + 1.0) * per_unit3 +
-               STREAM_K_FIXUP_US * (tile_n / 128) * (sharers / 2.0);
+        return LAUNCH_US + kb_each * per_kb(g) + (static_cast<double>(tiles) / g + 1.0) * PER_UNIT[kind] +
+               2.93 * (tile_n / 128) * (sharers / 2.0);
     }
     const int units = tiles * splits;
     if (dm.sm_count < cg || (mode == 2 && dm.max_clusters[splits] < 1)) return 1e300;   // cannot run on this device
-    const int waves = (mode == 2) ? ceil_div(tiles, dm.max_clusters[splits]) : ceil_div(units, dm.sm_count / cg);
-    const double per_kb = (cg == 2) ? 0.505 : (tile_n == 256 ? 0.53 : 0.44);
-    const double per_unit = (cg == 2) ? 1.40 : (tile_n == 256 ? 1.2 : 0.35);
-    double cost = 3.5 + waves * (ceil_div(KB, splits) * per_kb + per_unit);
+    const int at_once = (mode == 2) ? dm.max_clusters[splits] : dm.sm_count / cg;       // tiles (mode 2) or units
+    const int waves = ceil_div((mode == 2) ? tiles : units, at_once);
+    const int running = ((mode == 2) ? tiles : units) < at_once ? ((mode == 2) ? tiles : units) : at_once;
+    double cost = LAUNCH_US + waves * (ceil_div(KB, splits) * per_kb(running * (mode == 2 ? splits : cg)) + PER_UNIT[kind]);
     if (splits > 1 && mode == 2) {
         // One CTA per (tile, K range), not persistent: a second wave of clusters pays the prologue and the
-        // reduction again, and nothing of it overlaps the wave before (measured on M = 16384 shapes).
-        const double overhead = (tile_n == 256 ? 3.0 : 2.0) + 0.5 * splits * (tile_n / 128);
-        cost += overhead + (waves - 1) * (overhead + 3.0);
+        // reduction again, and nothing of it overlaps the wave before.
+        const double overhead = (tile_n == 256 ? 5.16 : 2.21) + 0.03 * splits * (tile_n / 128);
+        cost += overhead + (waves - 1) * (overhead + 4.13);
     } else if (splits > 1) {
-        // (pair tiles through the workspace measured 1.5 % slower than single-CTA tiles on 1024 x 1536 x 7168: + 1 us)
-        const double overhead = 3.5 + 1.0 * splits * (tile_n / 128) + (cg == 2 ? 1.0 : 0.0);
-        cost += (waves > 1) ? 2.0 * overhead : overhead;
+        const double overhead = 2.15 + 1.1 * splits * (tile_n / 128);
+        cost += (waves > 1) ? 4.0 * overhead : overhead;
     }
     return cost;
 }
@@ -288,13 +289,14 @@ static Config choose_config(const DeviceModel& dm, int M, int N, int K, int path
     // short K: the tile's partial sums stay in TMEM (mode 4), a member of the mn_large family (K is not cut)
     if (tile_n & FP8BS_SHORT_K) return Config{FP8BS_PATH_MN_LARGE, 256, 1, 1, 4, 0};
     if (KB <= 2 && path != FP8BS_PATH_MN_SMALL && splits <= 1 && !force_ws && !force_sk && want_tile == 0) {
-        // Measured on a B200: 5-6 % faster than the full-K kernel at K = 128 and, at K = 256, up to about three tiles
-        // per SM (1024 x 7168 x 256, 1.5 per SM: 7.20 against 7.64 us; 2048 x 7168 x 256, 3.0: 11.1 against 11.4);
-        // with more tiles the store path of the SMs sets the pace and the full-K kernel, which overlaps the MMAs of
-        // a tile with the scaling of the one before, is ahead (3072 x 7168 x 256, 4.5 per SM: 14.1 against 14.9 us;
-        // 6144 x 7168 x 256, 9.1: 23.7 against 24.4).
+        // 256-wide single-CTA tiles, the answer fp8bs_select_path has always given for such K (with many tiles the pair is
+        // 7-9 % ahead: 6144 x 7168 x 256 18.8 us).  Of their two kernels, on a B200, this one is 1-7 % faster than the full-K
+        // kernel with few tiles per SM (1104 x 3344 x 256 5.61 against 5.88 us, 2144 x 112 x 128 3.81 against 4.05, 1024 x
+        // 7168 x 256 7.00 against 7.02); with more the store path of the SMs sets the pace and the full-K kernel, which
+        // overlaps the MMAs of a tile with the scaling of the one before, is ahead (2528 x 4496 x 256, 2.4 per SM: 9.06
+        // against 9.70; 6144 x 7168 x 256, 9.1: 20.7 against 22.2).
         const int tiles = ceil_div(M, 128) * ceil_div(N, 256);
-        if (KB == 1 || tiles <= SHORT_K_MAX_WAVES * dm.sm_count) return Config{FP8BS_PATH_MN_LARGE, 256, 1, 1, 4, 0};
+        return Config{FP8BS_PATH_MN_LARGE, 256, 1, 1, (KB == 1 || tiles <= SHORT_K_MAX_WAVES * dm.sm_count) ? 4 : 0, 0};
     }
     // stream-K: a member of the mn_small family (it cuts K), chosen when it is asked for or when the caller left
     // both path and splits open
