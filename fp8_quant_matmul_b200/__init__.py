@@ -17,6 +17,7 @@ from .api import (  # noqa: F401
     SPLIT_WORKSPACE,
     STREAM_K,
     SHORT_K,
+    SMALL_M,
     gemm,
     gemm_ref,
     gemm_mn_small_static,

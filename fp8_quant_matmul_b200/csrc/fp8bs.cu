@@ -3,6 +3,7 @@
 // reference's gemmGPU wrapper and its geometry switch (check.cu:51-130).
 #include "../../include/fp8bs.h"
 #include "gemm_kernel.cuh"
+#include "gemm_small_m.cuh"
 
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -101,6 +102,13 @@ static int prepare_kernel()
     return FP8BS_OK;
 }
 
+template <int T>
+static int prepare_small_m()
+{
+    CUDA_TRY(cudaFuncSetAttribute(gemm_small_m_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, SmallMCfg<T>::SMEM_BYTES));
+    return FP8BS_OK;
+}
+
 // One-time set-up for the current device: capability check, kernel attributes, driver
 // entry point for tensor-map encoding (looked up at run time so that the library has no
 // link-time dependency on libcuda and loads on a machine without a driver).
@@ -138,7 +146,8 @@ static int device_setup(DeviceInfo** out)
             (rc = prepare_kernel<256, 1, 1>()) || (rc = prepare_kernel<256, 2, 1>()) ||
             (rc = prepare_kernel<128, 1, 2>()) || (rc = prepare_kernel<256, 1, 2>()) ||
             (rc = prepare_kernel<128, 1, 3>()) || (rc = prepare_kernel<256, 1, 3>()) ||
-            (rc = prepare_kernel<256, 1, 4>())) {
+            (rc = prepare_kernel<256, 1, 4>()) || (rc = prepare_small_m<16>()) ||
+            (rc = prepare_small_m<32>()) || (rc = prepare_small_m<64>())) {
             d.status = rc;
             return rc;
         }
@@ -201,7 +210,8 @@ struct Config {
     int cg;       // 1: a CTA owns 128 rows of a tile; 2: a pair of CTAs owns 256 rows
     int mode;     // 0 full K; 1 split-K reduced through a workspace; 2 split-K reduced inside a cluster;
                   // 3 stream-K: the K blocks of all tiles dealt out evenly over `ctas` CTAs; 4 short K (K <= 256):
-                  // full K with both K blocks of a tile resident in TMEM
+                  // full K with both K blocks of a tile resident in TMEM; 5 few rows (M <= 64): K cut over the CTAs of
+                  // a cluster, see gemm_small_m.cuh
     int ctas;     // mode 3 only
 };
 
@@ -211,6 +221,28 @@ static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
 // Stream-K grid: every SM, but at least 4 K blocks per CTA.  Never more CTAs than SMs: a CTA waits (bounded) for
 // partial tiles of CTAs that must therefore be running at the same time.
+constexpr int SMALL_M_MAX = 64;
+
+// Mode 5: K is cut over as many CTAs as there are SMs to read B with (tiles are 128 columns wide).  Measured with 1, 2, 3, ..
+// splits: 16 x 7168 x 2304 (56 tiles) 9.8, 7.9, 8.8 (168 CTAs: some SMs get two), 7.85 us; 16 x 1536 x 7168 (12 tiles) 22.2, 12.7,
+// 9.5, .., 6.2 with 8; 32 x 4096 x 2048 (32 tiles) 9.9, 7.5, 6.7, 6.2.  Up to four K blocks the reduction costs more than it
+// saves: 16 x 4608 x 256 2.9, 3.6; 32 x 7168 x 512 4.5, 5.1.  With long K (16 K blocks per CTA and more) two CTAs per SM keep
+// more loads in flight: 16 x 7168 x 7168 16.0 with 2 splits, 14.0 with 4.
+static Config small_m_config(const DeviceModel& dm, int N, int K, int splits)
+{
+    const int tiles = ceil_div(N, 128), KB = K / 128;
+    int s = splits;
+    if (s == 0) {
+        s = KB <= 4 ? 1 : dm.sm_count / tiles;
+        if (s >= 1 && KB / s >= 16 && 4 * tiles * s <= 7 * dm.sm_count) s *= 2;
+        if (s > MAX_CLUSTER_SPLITS) s = MAX_CLUSTER_SPLITS;
+        if (s > KB) s = KB;
+        while (s > 1 && dm.max_clusters[s] < 1) --s;
+        if (s < 1) s = 1;
+    }
+    return Config{s > 1 ? FP8BS_PATH_MN_SMALL : FP8BS_PATH_MN_LARGE, 128, s, 1, 5, 0};
+}
+
 static int stream_k_ctas(int tiles, int KB, int sm_count)
 {
     const long long total = static_cast<long long>(tiles) * KB;
@@ -283,9 +315,11 @@ static Config choose_config(const DeviceModel& dm, int M, int N, int K, int path
     const int KB = K / 128;
     const bool force_ws = (tile_n & FP8BS_SPLIT_WORKSPACE) != 0;
     const bool force_sk = (tile_n & FP8BS_STREAM_K) != 0;
-    const int want_tile = tile_n & ~(FP8BS_SPLIT_WORKSPACE | FP8BS_STREAM_K | FP8BS_SHORT_K);
+    const int want_tile = tile_n & ~(FP8BS_SPLIT_WORKSPACE | FP8BS_STREAM_K | FP8BS_SHORT_K | FP8BS_SMALL_M);
     Config best{FP8BS_PATH_MN_LARGE, 128, 1, 1, 0, 0};
     double best_cost = 1e300;
+    if (tile_n & FP8BS_SMALL_M) return small_m_config(dm, N, K, splits);
+    if (M <= SMALL_M_MAX && path == FP8BS_PATH_AUTO && splits == 0 && tile_n == 0) return small_m_config(dm, N, K, 0);
     // short K: the tile's partial sums stay in TMEM (mode 4), a member of the mn_large family (K is not cut)
     if (tile_n & FP8BS_SHORT_K) return Config{FP8BS_PATH_MN_LARGE, 256, 1, 1, 4, 0};
     if (KB <= 2 && path != FP8BS_PATH_MN_SMALL && splits <= 1 && !force_ws && !force_sk && want_tile == 0) {
@@ -361,10 +395,12 @@ static int check_args(int M, int N, int K, int n0, int n_total, int path, int sp
     if (splits < 0 || splits > K / 128 || splits > MAX_SPLITS) return FP8BS_ERR_ARG;
     if (path == FP8BS_PATH_MN_LARGE && splits > 1) return FP8BS_ERR_ARG;
     {
-        const int t = tile_n & ~(FP8BS_SPLIT_WORKSPACE | FP8BS_STREAM_K | FP8BS_SHORT_K);
+        const int t = tile_n & ~(FP8BS_SPLIT_WORKSPACE | FP8BS_STREAM_K | FP8BS_SHORT_K | FP8BS_SMALL_M);
         if (t != 0 && t != 128 && t != 256 && t != (256 | FP8BS_TILE_PAIR)) return FP8BS_ERR_ARG;
         if ((tile_n & FP8BS_SHORT_K) && ((t != 0 && t != 256) || (tile_n & (FP8BS_SPLIT_WORKSPACE | FP8BS_STREAM_K)) ||
                                          splits > 1 || path == FP8BS_PATH_MN_SMALL || K > 256))
+            return FP8BS_ERR_ARG;
+        if ((tile_n & FP8BS_SMALL_M) && (tile_n != FP8BS_SMALL_M || M > SMALL_M_MAX || splits > MAX_CLUSTER_SPLITS))
             return FP8BS_ERR_ARG;
         if ((tile_n & FP8BS_STREAM_K) && ((tile_n & (FP8BS_TILE_PAIR | FP8BS_SPLIT_WORKSPACE)) || splits > 1 ||
                                           path == FP8BS_PATH_MN_LARGE))
@@ -388,6 +424,24 @@ static int encode_operand_map(CUtensorMap* tm, const void* base, int mn, int K)
     const CUresult r = g_encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides,
                                       box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        tl_last_cuda_error = static_cast<int>(r);
+        return FP8BS_ERR_CUDA;
+    }
+    return FP8BS_OK;
+}
+
+// A for the kernel of few rows: box = `width` rows (32 or 64 bytes, swizzled over that width) x 128 k.
+static int encode_few_rows_map(CUtensorMap* tm, const void* base, int M, int K, int width)
+{
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(M), static_cast<cuuint64_t>(K)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(M)};
+    const cuuint32_t box[2] = {static_cast<cuuint32_t>(width), 128u};
+    const cuuint32_t estr[2] = {1u, 1u};
+    const CUresult r = g_encode_tiled(tm, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
+                                      CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                      width == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B,
+                                      CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) {
         tl_last_cuda_error = static_cast<int>(r);
         return FP8BS_ERR_CUDA;
@@ -431,6 +485,32 @@ struct TensorMaps {
     CMaps C;
 };
 
+// `Kernel` with clusters of `cluster` CTAs, as a programmatic dependent of the kernel before it in the stream: it does its
+// set-up, then waits for that kernel (griddepcontrol.wait) before it touches global memory, which hides launch latency and
+// set-up behind that kernel's tail.
+template <class Kernel, class... Args>
+static int launch_clusters(Kernel kernel, int ctas, int cluster, int threads, int smem, cudaStream_t stream, const Args&... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(ctas), 1, 1);
+    cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
+    cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = g_use_pdl ? 2 : 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, args...);
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    CUDA_TRY(e);
+    return FP8BS_OK;
+}
+
 template <int BN, int CG, int MODE>
 static int launch(const TensorMaps& tm, const GemmParams& p, int sm_count, cudaStream_t stream)
 {
@@ -439,30 +519,21 @@ static int launch(const TensorMaps& tm, const GemmParams& p, int sm_count, cudaS
     int groups = units < sm_count / CG ? units : sm_count / CG;    // tile walkers: CTAs or CTA pairs
     if (MODE == 2) groups = units;                                  // one CTA per (tile, K range); a cluster per tile
     if (MODE == 3) groups = stream_k_ctas(p.m_tiles * p.n_tiles, p.K / 128, sm_count);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(groups * CG), 1, 1);
-    cfg.blockDim = dim3(Cfg::THREADS, 1, 1);
-    cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (MODE == 2) ? static_cast<unsigned>(p.splits) : CG;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    // The kernel does its set-up, then waits for the previous kernel of the stream (griddepcontrol.wait) before it
-    // touches global memory: letting it start early hides launch latency and set-up behind that kernel's tail.
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = g_use_pdl ? 2 : 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_kernel<BN, CG, MODE>, tm.A, tm.B, tm.C, p);
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    CUDA_TRY(e);
-    return FP8BS_OK;
+    return launch_clusters(gemm_kernel<BN, CG, MODE>, groups * CG, MODE == 2 ? p.splits : CG, Cfg::THREADS, Cfg::SMEM_BYTES, stream,
+                           tm.A, tm.B, tm.C, p);
+}
+
+template <int T>
+static int launch_small_m(const TensorMaps& tm, const GemmParams& p, cudaStream_t stream)
+{
+    using Cfg = SmallMCfg<T>;
+    return launch_clusters(gemm_small_m_kernel<T>, p.n_tiles * p.splits, p.splits, Cfg::THREADS, Cfg::SMEM_BYTES, stream, tm.A, tm.B, p);
 }
 
 static int launch_config(const Config& c, const TensorMaps& tm, const GemmParams& p, int sm_count, cudaStream_t st)
 {
+    if (c.mode == 5)
+        return p.M <= 16 ? launch_small_m<16>(tm, p, st) : p.M <= 32 ? launch_small_m<32>(tm, p, st) : launch_small_m<64>(tm, p, st);
     if (c.mode == 3)
         return c.tile_n == 256 ? launch<256, 1, 3>(tm, p, sm_count, st) : launch<128, 1, 3>(tm, p, sm_count, st);
     if (c.mode == 2)
@@ -519,12 +590,12 @@ static int gemm_impl(const void* A, const void* B, const float* a_scale, const f
     if (dev_rc) return dev_rc;
 
     TensorMaps tm{};
-    if ((rc = encode_operand_map(&tm.A, A, M, K))) return rc;
+    if ((rc = cfg.mode == 5 ? encode_few_rows_map(&tm.A, A, M, K, M <= 32 ? 32 : 64) : encode_operand_map(&tm.A, A, M, K))) return rc;
     if ((rc = encode_operand_map(&tm.B, B, N, K))) return rc;
     if (dests) {
         for (int d = 0; d < n_dest; ++d)
             if ((rc = encode_c_map(&tm.C.m[d], static_cast<__nv_bfloat16*>(dests[d]) + n0, M, N, n_total))) return rc;
-    } else if ((rc = encode_c_map(&tm.C.m[0], C, M, N, N))) return rc;
+    } else if (cfg.mode != 5 && (rc = encode_c_map(&tm.C.m[0], C, M, N, N))) return rc;
 
     GemmParams p;
     p.a_scale = a_scale;
@@ -779,7 +850,7 @@ int fp8bs_select_path(int M, int N, int K, int* splits, int* tile_n)
     if (rc) return rc;
     const Config c = choose_config(host_model(), M, N, K, FP8BS_PATH_AUTO, 0, 0);
     if (splits) *splits = c.splits;
-    if (tile_n) *tile_n = c.tile_n | (c.cg == 2 ? FP8BS_TILE_PAIR : 0) | (c.mode == 1 ? FP8BS_SPLIT_WORKSPACE : 0) | (c.mode == 4 ? FP8BS_SHORT_K : 0) |
+    if (tile_n) *tile_n = c.tile_n | (c.cg == 2 ? FP8BS_TILE_PAIR : 0) | (c.mode == 1 ? FP8BS_SPLIT_WORKSPACE : 0) | (c.mode == 4 ? FP8BS_SHORT_K : 0) | (c.mode == 5 ? FP8BS_SMALL_M : 0) |
                           (c.mode == 3 ? FP8BS_STREAM_K : 0);
     return c.path;
 }
@@ -791,12 +862,12 @@ int fp8bs_select_path_sms(int M, int N, int K, int sm_count, int* splits, int* t
     if (sm_count < 1) return FP8BS_ERR_ARG;
     const Config c = choose_config(scaled_model(sm_count), M, N, K, FP8BS_PATH_AUTO, 0, 0);
     if (splits) *splits = c.splits;
-    if (tile_n) *tile_n = c.tile_n | (c.cg == 2 ? FP8BS_TILE_PAIR : 0) | (c.mode == 1 ? FP8BS_SPLIT_WORKSPACE : 0) | (c.mode == 4 ? FP8BS_SHORT_K : 0) |
+    if (tile_n) *tile_n = c.tile_n | (c.cg == 2 ? FP8BS_TILE_PAIR : 0) | (c.mode == 1 ? FP8BS_SPLIT_WORKSPACE : 0) | (c.mode == 4 ? FP8BS_SHORT_K : 0) | (c.mode == 5 ? FP8BS_SMALL_M : 0) |
                           (c.mode == 3 ? FP8BS_STREAM_K : 0);
     if (ctas) {
         // CTAs that have to be resident together: stream-K's whole grid, one cluster for the cluster reduction,
         // otherwise none (the tile walkers never wait on one another)
-        *ctas = (c.mode == 3) ? c.ctas : (c.mode == 2 ? c.splits : 0);
+        *ctas = (c.mode == 3) ? c.ctas : (c.mode == 2 || (c.mode == 5 && c.splits > 1) ? c.splits : 0);
     }
     return c.path;
 }

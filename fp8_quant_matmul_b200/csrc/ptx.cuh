@@ -176,6 +176,20 @@ __device__ __forceinline__ void cluster_sync()
 {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same barrier in two halves: arrive early, wait where the peers' arrival matters.
+__device__ __forceinline__ void cluster_arrive()
+{
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait()
+{
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// 4 bytes into the shared memory of any CTA of the cluster (address from mapa).
+__device__ __forceinline__ void st_shared_cluster_f32(uint32_t cluster_addr, float v)
+{
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_addr), "f"(v) : "memory");
+}
 // 16 bytes from the shared memory of any CTA of the cluster (address from mapa).
 __device__ __forceinline__ float4 ld_shared_cluster_v4(uint32_t cluster_addr)
 {
@@ -303,6 +317,19 @@ __device__ __forceinline__ void ld_shared_f32(uint32_t addr, float& x)
     asm volatile("ld.shared.f32 %0, [%1];" : "=f"(x) : "r"(addr) : "memory");
 }
 
+// Two pairs of floats, each as the operand of fma.rn.f32x2.
+__device__ __forceinline__ void ld_shared_v2_b64(uint32_t addr, unsigned long long& x, unsigned long long& y)
+{
+    asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(x), "=l"(y) : "r"(addr) : "memory");
+}
+// (a.lo * b.lo + c.lo, a.hi * b.hi + c.hi)
+__device__ __forceinline__ unsigned long long fma_f32x2(unsigned long long a, unsigned long long b, unsigned long long c)
+{
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
 // 64 columns from TMEM, complete on return (load and wait in one statement).
 __device__ __forceinline__ void tmem_ld_x64_sync(uint32_t taddr, uint32_t (&v)[64])
 {
@@ -334,16 +361,20 @@ __device__ __forceinline__ void tmem_ld_2x64_sync(uint32_t taddr_a, uint32_t tad
 // along K, `lbo` the byte distance between consecutive 128-wide slabs along M/N.
 //   bits [0,14)  start address >> 4      bits [16,30) lbo >> 4     bits [32,46) sbo >> 4
 //   bits [46,48) descriptor version (1 on sm_100)      bits [61,64) swizzle (2 = 128 B)
-__device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr, uint32_t lbo,
-                                                         uint32_t sbo)
+// `swizzle` 4 (64 B) and 6 (32 B): the same with rows and atoms of that width.
+__device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t lbo, uint32_t sbo, uint32_t swizzle)
 {
     uint64_t d = 0;
     d |= static_cast<uint64_t>((smem_addr >> 4) & 0x3FFFu);
     d |= static_cast<uint64_t>((lbo >> 4) & 0x3FFFu) << 16;
     d |= static_cast<uint64_t>((sbo >> 4) & 0x3FFFu) << 32;
     d |= static_cast<uint64_t>(1) << 46;
-    d |= static_cast<uint64_t>(2) << 61;
+    d |= static_cast<uint64_t>(swizzle) << 61;
     return d;
+}
+__device__ __forceinline__ uint64_t make_smem_desc_sw128(uint32_t smem_addr, uint32_t lbo, uint32_t sbo)
+{
+    return make_smem_desc(smem_addr, lbo, sbo, 2u);
 }
 // Instruction descriptor for kind::f8f6f4: e4m3 x e4m3 -> fp32, both operands MN-major.
 //   [4,6) D format (1 = f32)  [7,10) A format (0 = e4m3)  [10,13) B format (0 = e4m3)
