@@ -371,6 +371,30 @@ static Config choose_config(const DeviceModel& dm, int M, int N, int K, int path
     return best;
 }
 
+// choose_config, remembered per thread for the last shapes asked about: pricing every configuration takes 0.5-1 us, as much
+// as encoding the tensor maps.  `device` is the device whose model `dm` is (its model never changes once it is set up), or -1
+// for the model of no device in particular.
+static Config plan(const DeviceModel& dm, int device, int M, int N, int K, int path, int splits, int tile_n)
+{
+    struct Entry {
+        int key[7];
+        Config cfg;
+        bool used;
+    };
+    constexpr int ENTRIES = 64;
+    static thread_local Entry table[ENTRIES];
+    const int key[7] = {device, M, N, K, path, splits, tile_n};
+    unsigned h = 2166136261u;
+    for (int v : key) h = (h ^ static_cast<unsigned>(v)) * 16777619u;
+    Entry& e = table[(h >> 16) % ENTRIES];
+    if (!e.used || std::memcmp(e.key, key, sizeof(key)) != 0) {
+        e.cfg = choose_config(dm, M, N, K, path, splits, tile_n);
+        std::memcpy(e.key, key, sizeof(key));
+        e.used = true;
+    }
+    return e.cfg;
+}
+
 static size_t config_workspace(int M, int N, const Config& c)
 {
     if (c.mode == 3)                                                 // flags + one partial tile per CTA
@@ -574,7 +598,7 @@ static int gemm_impl(const void* A, const void* B, const float* a_scale, const f
     DeviceInfo* dev = nullptr;
     const int dev_rc = device_setup(&dev);
     const DeviceModel dm = (dev_rc == FP8BS_OK) ? dev->model : kB200Model;
-    Config cfg = choose_config(dm, M, N, K, path, splits, tile_n);
+    Config cfg = plan(dm, dev_rc == FP8BS_OK ? static_cast<int>(dev - g_dev) : -1, M, N, K, path, splits, tile_n);
     if (dests && cfg.mode == 2) return FP8BS_ERR_ARG;       // the cluster reduction stores C itself, to one buffer
     if (cfg.mode == 1 || cfg.mode == 3) {
         const size_t need = config_workspace(M, N, cfg);
