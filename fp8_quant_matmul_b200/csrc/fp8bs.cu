@@ -4,6 +4,7 @@
 #include "../../include/fp8bs.h"
 #include "gemm_kernel.cuh"
 #include "gemm_small_m.cuh"
+#include "quantize.cuh"
 
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -109,6 +110,13 @@ static int prepare_small_m()
     return FP8BS_OK;
 }
 
+template <bool BLOCK_SCALE>
+static int prepare_quantize()
+{
+    CUDA_TRY(cudaFuncSetAttribute(quantize_bf16_kernel<BLOCK_SCALE>, cudaFuncAttributeMaxDynamicSharedMemorySize, QUANTIZE_BF16_SMEM));
+    return FP8BS_OK;
+}
+
 // One-time set-up for the current device: capability check, kernel attributes, driver
 // entry point for tensor-map encoding (looked up at run time so that the library has no
 // link-time dependency on libcuda and loads on a machine without a driver).
@@ -147,7 +155,8 @@ static int device_setup(DeviceInfo** out)
             (rc = prepare_kernel<128, 1, 2>()) || (rc = prepare_kernel<256, 1, 2>()) ||
             (rc = prepare_kernel<128, 1, 3>()) || (rc = prepare_kernel<256, 1, 3>()) ||
             (rc = prepare_kernel<256, 1, 4>()) || (rc = prepare_small_m<16>()) ||
-            (rc = prepare_small_m<32>()) || (rc = prepare_small_m<64>())) {
+            (rc = prepare_small_m<32>()) || (rc = prepare_small_m<64>()) ||
+            (rc = prepare_quantize<false>()) || (rc = prepare_quantize<true>())) {
             d.status = rc;
             return rc;
         }
@@ -513,10 +522,10 @@ struct TensorMaps {
 // set-up, then waits for that kernel (griddepcontrol.wait) before it touches global memory, which hides launch latency and
 // set-up behind that kernel's tail.
 template <class Kernel, class... Args>
-static int launch_clusters(Kernel kernel, int ctas, int cluster, int threads, int smem, cudaStream_t stream, const Args&... args)
+static int launch_grid(Kernel kernel, dim3 grid, int cluster, int threads, int smem, cudaStream_t stream, const Args&... args)
 {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(ctas), 1, 1);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(static_cast<unsigned>(threads), 1, 1);
     cfg.dynamicSmemBytes = static_cast<size_t>(smem);
     cfg.stream = stream;
@@ -533,6 +542,12 @@ static int launch_clusters(Kernel kernel, int ctas, int cluster, int threads, in
     g_launches.fetch_add(1, std::memory_order_relaxed);
     CUDA_TRY(e);
     return FP8BS_OK;
+}
+
+template <class Kernel, class... Args>
+static int launch_clusters(Kernel kernel, int ctas, int cluster, int threads, int smem, cudaStream_t stream, const Args&... args)
+{
+    return launch_grid(kernel, dim3(static_cast<unsigned>(ctas), 1, 1), cluster, threads, smem, stream, args...);
 }
 
 template <int BN, int CG, int MODE>
@@ -730,10 +745,6 @@ __host__ __device__ inline uint8_t float_to_e4m3fn_rne(float x)
     if (be > 15u || (be == 15u && q == 7u)) return sign | 0x7E;
     return sign | static_cast<uint8_t>((be << 3) | q);
 }
-
-}  // namespace fp8bs
-#include "quantize.cuh"
-namespace fp8bs {
 
 __global__ void convert_float_to_e4m3fn_kernel(const float* __restrict__ in, uint8_t* __restrict__ out, size_t n)
 {
@@ -1303,21 +1314,29 @@ static int quantize_impl(bool block, const void* X, int x_is_bf16, void* out, fl
     DeviceInfo* dev = nullptr;
     const int rc = device_setup(&dev);
     if (rc) return rc;
-    const dim3 grid(ceil_div(rows, 128), K / 128), blk(256);
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     uint8_t* o = static_cast<uint8_t*>(out);
-    if (x_is_bf16) {
-        const __nv_bfloat16* x = static_cast<const __nv_bfloat16*>(X);
-        if (block) quantize_kernel<true, __nv_bfloat16><<<grid, blk, 0, st>>>(x, o, scale_out, rows, K, fp8_max);
-        else quantize_kernel<false, __nv_bfloat16><<<grid, blk, 0, st>>>(x, o, scale_out, rows, K, fp8_max);
-    } else {
+    const dim3 grid(ceil_div(rows, 128), K / 128, 1);
+    if (!x_is_bf16) {
         const float* x = static_cast<const float*>(X);
-        if (block) quantize_kernel<true, float><<<grid, blk, 0, st>>>(x, o, scale_out, rows, K, fp8_max);
-        else quantize_kernel<false, float><<<grid, blk, 0, st>>>(x, o, scale_out, rows, K, fp8_max);
+        return launch_grid(block ? quantize_f32_kernel<true> : quantize_f32_kernel<false>, grid, 1, 256, 0, st, x, o, scale_out, rows, K,
+                           fp8_max);
     }
-    g_launches.fetch_add(1, std::memory_order_relaxed);
-    CUDA_TRY(cudaGetLastError());
-    return FP8BS_OK;
+    CUtensorMap tm;                                  // X as a 2-D tensor {K, rows}; box = one 128 x 128 tile
+    const cuuint64_t dims[2] = {static_cast<cuuint64_t>(K), static_cast<cuuint64_t>(rows)};
+    const cuuint64_t strides[1] = {static_cast<cuuint64_t>(K) * 2};
+    const cuuint32_t box[2] = {128u, 128u}, estr[2] = {1u, 1u};
+    const CUresult r = g_encode_tiled(&tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(X), dims, strides, box, estr,
+                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        tl_last_cuda_error = static_cast<int>(r);
+        return FP8BS_ERR_CUDA;
+    }
+    const long long tiles = static_cast<long long>(grid.x) * grid.y, most = static_cast<long long>(dev->sm_count) * QUANTIZE_BF16_CTAS;
+    return launch_grid(block ? quantize_bf16_kernel<true> : quantize_bf16_kernel<false>,
+                       dim3(static_cast<unsigned>(tiles < most ? tiles : most), 1, 1), 1, 256, QUANTIZE_BF16_SMEM, st, tm, o, scale_out, rows,
+                       K, fp8_max, dev->status_ptr);
 }
 
 int fp8bs_quantize_rowwise(const void* X, int x_is_bf16, void* A_out, float* a_scale_out, int M, int K, float fp8_max,
