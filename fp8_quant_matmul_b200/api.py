@@ -63,6 +63,7 @@ _SIGS = {
     "fp8bs_float_to_e4m3fn": (_c.c_uint8, [_c.c_float]),
     "fp8bs_e4m3fn_to_float": (_c.c_float, [_c.c_uint8]),
     "fp8bs_fnuz_to_fn_device": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_size_t, _c.c_void_p, _c.c_void_p]),
+    "fp8bs_fnuz_to_fn_device_sync": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_size_t, _c.POINTER(_c.c_uint), _c.c_void_p]),
     "fp8bs_fnuz_to_fn": (_c.c_int, [_c.c_void_p, _c.c_void_p, _c.c_size_t, _c.POINTER(_c.c_size_t)]),
 }
 
@@ -178,14 +179,12 @@ def fnuz_to_fn(src):
 
 def fnuz_to_fn_device(src, dst=None):
     """Re-encode a CUDA uint8 tensor of e4m3fnuz bytes as e4m3fn bytes; returns (dst, number of inexact bytes)."""
-    torch = _torch()
     if dst is None:
-        dst = torch.empty_like(src)
-    count = torch.zeros(1, dtype=torch.int32, device=src.device)
-    stream = torch.cuda.current_stream(src.device).cuda_stream
-    _check(lib().fp8bs_fnuz_to_fn_device(dst.data_ptr(), src.data_ptr(), src.numel(), count.data_ptr(), stream),
-           "fp8bs_fnuz_to_fn_device")
-    return dst, int(count.item())
+        dst = _torch().empty_like(src)
+    count = _c.c_uint(0)
+    _check(lib().fp8bs_fnuz_to_fn_device_sync(dst.data_ptr(), src.data_ptr(), src.numel(), _c.byref(count),
+                                              _stream(src.get_device())), "fp8bs_fnuz_to_fn_device_sync")
+    return dst, count.value
 
 
 # ---------------------------------------------------------------- the operator ---------
