@@ -276,19 +276,24 @@ static int stream_k_ctas(int tiles, int KB, int sm_count)
 
 
 // Estimated run time of a configuration in microseconds.  The constants are a least-squares fit to a sweep of every
-// configuration over 85 shapes on a B200 (the 18 benchmark shapes and random ones, M 80..16384, N 64..7168, K 128..7168, cold
-// L2, launches back to back); choosing by it costs 0.8 % on average against the best configuration of each shape, 16 % at
-// most (the constants before it, fitted to slower kernels, 3.7 %).  The overheads of the two split-K forms are 1.5 and 0.6 us above
-// the fit, which settles near ties for the kernel that does not cut K.  Per 128-K block of a work unit 0.23 us (128-wide tile), 0.45 (256-wide), 0.41 (256 x 256 pair), and up to 27 % / 15 %
-// / 0 % more the more SMs take part; per work unit 1.9 / 1.5 / 1.5 us (tile switch, epilogue), 3 us per launch.
+// configuration over 94 shapes on a B200 (the 18 benchmark shapes, random and ragged ones, M 80..16384, N 64..7168, K 128..7168,
+// cold L2, launches back to back); choosing by it costs 0.3 % on average against the best configuration of each shape, 6 % at
+// most.  A 128-K block of a work unit takes the larger of two times:
+//   its MMAs, promotion and hand-over: 0.24 us (128-wide tile), 0.46 (256-wide), 0.37 (256 x 256 pair), and up to 22 / 10 / 7 %
+//   more the more SMs take part;
+//   its loads: 0.24 / 0.34 / 0.25 us, and 91 % more where the rows of an operand's boxes do not start on 32-byte sectors
+//   (M or N an odd multiple of 16: 1968 x 496 x 7040 takes 32.4 us on 128-wide tiles, 2048 x 512 x 7168 17.5).
+// Per work unit 1.9 / 2.0 / 2.4 us (tile switch, epilogue), 1.9 us per launch.
 // Examples, 128-wide / 256-wide / pair: 1024 x 7168 x 2304 23.1 / 22.9 / 20.0 us, 128 x 7168 x 2304 9.2 / 13.3 / 11.8, 1024 x
 // 1536 x 7168 18.7 / 28.0 / 23.9 (best with K cut: 20.7).
-//   split-K through a workspace: 2.15 us + 1.1 us per split and 128 columns for the partial-sum round trip, four times
-//   that when a CTA has to walk more than one unit (the last-arriver reduction then delays the next unit);
+//   split-K through a workspace: 1.7 us + 1.0 us per split and 128 columns for the partial-sum round trip (4.1 us more
+//   for pairs), three times that when a CTA has to walk more than one unit (the last-arriver reduction then delays the
+//   next unit);
 //   split-K inside a cluster: one CTA per (tile, K range); the number of clusters that fit on the GPU at once is
-//   cudaOccupancyMaxActiveClusters for this kernel's footprint (one CTA per SM); overhead 2.2 us (5.2 us for 256-wide
-//   tiles), paid again with 4.1 us of prologue by every further wave of clusters;
-//   stream-K: 2.9 us per 128 columns of tile width for the hand-over of partial tiles, times half the number of CTAs that
+//   cudaOccupancyMaxActiveClusters for this kernel's footprint (one CTA per SM); overhead 2.6 us (5.1 us for 256-wide
+//   tiles; 0.4 above the fit, which settles near ties for the kernel that does not cut K), paid again with 2.8 us of
+//   prologue by every further wave of clusters;
+//   stream-K: 3.2 us per 128 columns of tile width for the hand-over of partial tiles, times half the number of CTAs that
 //   share a tile (the finishing CTA reads the others' one after the other).
 // Mode 4 (K <= 256, partial sums resident in TMEM) is chosen by rule, see choose_config.
 constexpr int SHORT_K_MAX_WAVES = 3;
@@ -297,10 +302,15 @@ static double config_cost(const DeviceModel& dm, int M, int N, int K, int tile_n
     const int KB = K / 128;
     const int tiles = ceil_div(M, 128 * cg) * ceil_div(N, tile_n);
     const int kind = (cg == 2) ? 2 : (tile_n == 256 ? 1 : 0);
-    static const double PER_KB[3] = {0.232, 0.452, 0.407}, CROWDING[3] = {0.274, 0.147, 0.0}, PER_UNIT[3] = {1.875, 1.529, 1.533};
-    constexpr double LAUNCH_US = 3.0;
+    static const double PER_KB[3] = {0.236, 0.455, 0.374}, CROWDING[3] = {0.218, 0.095, 0.067}, PER_UNIT[3] = {1.919, 1.979, 2.419};
+    static const double LOAD_KB[3] = {0.239, 0.344, 0.246}, A_SHARE[3] = {0.5, 1.0 / 3.0, 0.5};     // of a K block's operand bytes
+    constexpr double LAUNCH_US = 1.9, OFF_SECTOR = 0.911;
+    const double off_sector = OFF_SECTOR * (A_SHARE[kind] * (M % 32 != 0) + (1.0 - A_SHARE[kind]) * (N % 32 != 0));
     // K block time when `ctas` CTAs are at work
-    auto per_kb = [&](int ctas) { return PER_KB[kind] * (1.0 + CROWDING[kind] * ctas / dm.sm_count); };
+    auto per_kb = [&](int ctas) {
+        const double work = PER_KB[kind] * (1.0 + CROWDING[kind] * ctas / dm.sm_count), load = LOAD_KB[kind] * (1.0 + off_sector);
+        return work > load ? work : load;
+    };
     if (mode == 3) {
         // every CTA: ceil(T / G) K blocks, its share of the tile switches, one partial-sum hand-over each way
         const int g = stream_k_ctas(tiles, KB, dm.sm_count);
@@ -309,7 +319,7 @@ static double config_cost(const DeviceModel& dm, int M, int N, int K, int tile_n
         // the CTA that finishes a tile reads the partial tile of every other CTA that worked on it, one after the other
         const double sharers = (kb_each < KB) ? (KB / kb_each + 1.0) : 2.0;
         return LAUNCH_US + kb_each * per_kb(g) + (static_cast<double>(tiles) / g + 1.0) * PER_UNIT[kind] +
-               2.93 * (tile_n / 128) * (sharers / 2.0);
+               3.24 * (tile_n / 128) * (sharers / 2.0);
     }
     const int units = tiles * splits;
     if (dm.sm_count < cg || (mode == 2 && dm.max_clusters[splits] < 1)) return 1e300;   // cannot run on this device
@@ -320,11 +330,11 @@ static double config_cost(const DeviceModel& dm, int M, int N, int K, int tile_n
     if (splits > 1 && mode == 2) {
         // One CTA per (tile, K range), not persistent: a second wave of clusters pays the prologue and the
         // reduction again, and nothing of it overlaps the wave before.
-        const double overhead = (tile_n == 256 ? 5.16 : 2.21) + 0.03 * splits * (tile_n / 128);
-        cost += overhead + (waves - 1) * (overhead + 4.13);
+        const double overhead = (tile_n == 256 ? 5.09 : 2.64) + 0.057 * splits * (tile_n / 128);
+        cost += overhead + (waves - 1) * (overhead + 2.77);
     } else if (splits > 1) {
-        const double overhead = 2.15 + 1.1 * splits * (tile_n / 128);
-        cost += (waves > 1) ? 4.0 * overhead : overhead;
+        const double overhead = 1.7 + 1.03 * splits * (tile_n / 128) + (cg == 2 ? 4.09 : 0.0);
+        cost += (waves > 1) ? 3.05 * overhead : overhead;
     }
     return cost;
 }
