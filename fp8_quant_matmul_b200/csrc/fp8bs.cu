@@ -14,6 +14,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <cstdint>
 #include <cstdlib>
 #include <mutex>
 #include <new>
@@ -342,7 +343,9 @@ static double config_cost(const DeviceModel& dm, int M, int N, int K, int tile_n
 // tile_n argument of the API: 0 = choose; 128 or 256 = tile width, one CTA per tile;
 // 256 | FP8BS_TILE_PAIR = 256 x 256 tile owned by a pair of CTAs; | FP8BS_SPLIT_WORKSPACE = reduce split-K partial
 // sums through the workspace even where the cluster reduction could be used.
-static Config choose_config(const DeviceModel& dm, int M, int N, int K, int path, int splits, int tile_n)
+// ws_limit: only configurations that need no more workspace than this (a mn_large answer to a mn_small question: there is none).
+static size_t config_workspace(int M, int N, const Config& c);
+static Config choose_config(const DeviceModel& dm, int M, int N, int K, int path, int splits, int tile_n, size_t ws_limit = SIZE_MAX)
 {
     const int KB = K / 128;
     const bool force_ws = (tile_n & FP8BS_SPLIT_WORKSPACE) != 0;
@@ -374,9 +377,10 @@ static Config choose_config(const DeviceModel& dm, int M, int N, int K, int path
             // through L2 (measured: 369 us against 186 us on 16384 x 1536 x 7168): only on request there.
             if (!force_sk && tiles > dm.sm_count) continue;
             const double c = config_cost(dm, M, N, K, tn, 1, 1, 3);
-            if (c < best_cost) {
+            const Config cand{FP8BS_PATH_MN_SMALL, tn, 1, 1, 3, stream_k_ctas(tiles, KB, dm.sm_count)};
+            if (c < best_cost && config_workspace(M, N, cand) <= ws_limit) {
                 best_cost = c;
-                best = Config{FP8BS_PATH_MN_SMALL, tn, 1, 1, 3, stream_k_ctas(tiles, KB, dm.sm_count)};
+                best = cand;
             }
         }
         if (force_sk) return best;
@@ -393,9 +397,10 @@ static Config choose_config(const DeviceModel& dm, int M, int N, int K, int path
                                         dm.max_clusters[s] > 0;
                 for (int mode = small ? 1 : 0; mode <= (cluster_ok ? 2 : (small ? 1 : 0)); ++mode) {
                     const double c = config_cost(dm, M, N, K, tn, s, cg, mode);
-                    if (c < best_cost) {
+                    const Config cand{small ? FP8BS_PATH_MN_SMALL : FP8BS_PATH_MN_LARGE, tn, s, cg, mode, 0};
+                    if (c < best_cost && config_workspace(M, N, cand) <= ws_limit) {
                         best_cost = c;
-                        best = Config{small ? FP8BS_PATH_MN_SMALL : FP8BS_PATH_MN_LARGE, tn, s, cg, mode, 0};
+                        best = cand;
                     }
                 }
             }
@@ -638,15 +643,22 @@ static int gemm_impl(const void* A, const void* B, const float* a_scale, const f
     const DeviceModel dm = (dev_rc == FP8BS_OK) ? dev->model : kB200Model;
     Config cfg = plan(dm, dev_rc == FP8BS_OK ? static_cast<int>(dev - g_dev) : -1, M, N, K, path, splits, tile_n);
     if (dests && cfg.mode == 2) return FP8BS_ERR_ARG;       // the cluster reduction stores C itself, to one buffer
-    if (cfg.mode == 1 || cfg.mode == 3) {
-        const size_t need = config_workspace(M, N, cfg);
-        const size_t half_tiles = (cfg.mode == 3) ? static_cast<size_t>(cfg.ctas)
-            : static_cast<size_t>(ceil_div(M, 128 * cfg.cg)) * cfg.cg * ceil_div(N, cfg.tile_n);
-        const bool fits = workspace && workspace_bytes >= need && half_tiles <= COUNTER_BYTES / sizeof(unsigned int) &&
-                          (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0;
-        if (!fits) {
-            if (path != FP8BS_PATH_AUTO || (tile_n & (FP8BS_STREAM_K | FP8BS_SPLIT_WORKSPACE))) return FP8BS_ERR_WORKSPACE;
+    const bool ws_usable = workspace && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0;
+    auto fits = [&](const Config& c) {
+        if (c.mode != 1 && c.mode != 3) return true;
+        const size_t half_tiles = (c.mode == 3) ? static_cast<size_t>(c.ctas)
+            : static_cast<size_t>(ceil_div(M, 128 * c.cg)) * c.cg * ceil_div(N, c.tile_n);
+        return ws_usable && workspace_bytes >= config_workspace(M, N, c) && half_tiles <= COUNTER_BYTES / sizeof(unsigned int);
+    };
+    if (!fits(cfg)) {
+        if (path == FP8BS_PATH_AUTO && !(tile_n & (FP8BS_STREAM_K | FP8BS_SPLIT_WORKSPACE))) {
             cfg = choose_config(dm, M, N, K, FP8BS_PATH_MN_LARGE, 1, tile_n);   // best full-K configuration
+        } else {
+            // with the number of splits left open, the best way to cut K that fits: which workspace suffices does not hang on
+            // the constants of the estimate
+            if (splits != 0) return FP8BS_ERR_WORKSPACE;
+            cfg = choose_config(dm, M, N, K, path, splits, tile_n, ws_usable ? workspace_bytes : 0);
+            if (cfg.path != FP8BS_PATH_MN_SMALL || !fits(cfg)) return FP8BS_ERR_WORKSPACE;
         }
     }
     if (dev_rc) return dev_rc;
@@ -864,8 +876,8 @@ int fp8bs_gemm_mn_small_static(const void* A, const void* B, const float* a_scal
     int rc = check_args(M, N, K, 0, N, FP8BS_PATH_MN_SMALL, splits, 0);
     if (rc) return rc;
     // refuse anything the built-in scratch cannot hold, before touching the device
-    const Config cfg = choose_config(host_model(), M, N, K, FP8BS_PATH_MN_SMALL, splits, FP8BS_SPLIT_WORKSPACE);
-    if (config_workspace(M, N, cfg) > STATIC_SCRATCH_BYTES) return FP8BS_ERR_WORKSPACE;
+    const Config cfg = choose_config(host_model(), M, N, K, FP8BS_PATH_MN_SMALL, splits, FP8BS_SPLIT_WORKSPACE, STATIC_SCRATCH_BYTES);
+    if (cfg.path != FP8BS_PATH_MN_SMALL || config_workspace(M, N, cfg) > STATIC_SCRATCH_BYTES) return FP8BS_ERR_WORKSPACE;
     DeviceInfo* dev = nullptr;
     rc = device_setup(&dev);                       // first call on a device: attribute set-up, no allocation
     if (rc) return rc;
