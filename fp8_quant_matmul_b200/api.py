@@ -179,6 +179,8 @@ def fnuz_to_fn(src):
 
 def fnuz_to_fn_device(src, dst=None):
     """Re-encode a CUDA uint8 tensor of e4m3fnuz bytes as e4m3fn bytes; returns (dst, number of inexact bytes)."""
+    if not src.is_cuda or (dst is not None and (not dst.is_cuda or dst.get_device() != src.get_device())):
+        raise ValueError("expected CUDA tensors on one device")
     if dst is None:
         dst = _torch().empty_like(src)
     count = _c.c_uint(0)
