@@ -4,7 +4,9 @@ Device memory, streams and (in the benchmark) torch.distributed come from PyTorc
 arithmetic happens in the library's CUDA kernels.
 """
 import ctypes
+import itertools
 import os
+import threading
 
 import numpy as np
 
@@ -46,6 +48,9 @@ _SIGS = {
     "fp8bs_workspace_bytes": (_c.c_size_t, [_c.c_int] * 3),
     "fp8bs_workspace_bytes_ex": (_c.c_size_t, [_c.c_int] * 6),
     "fp8bs_workspace_init": (_c.c_int, [_c.c_void_p, _c.c_size_t, _c.c_void_p]),
+    "fp8bs_capture_id": (_c.c_int, [_c.c_void_p, _c.POINTER(_c.c_ulonglong)]),
+    "fp8bs_capture_hold": (_c.c_int, [_c.c_void_p, _c.c_ulonglong]),
+    "fp8bs_capture_released": (_c.c_int, [_c.POINTER(_c.c_ulonglong), _c.c_int]),
     "fp8bs_last_device_status": (_c.c_int, [_c.c_void_p, _c.POINTER(_c.c_uint)]),
     "fp8bs_selftest_wait_timeout": (_c.c_int, [_c.c_void_p]),
     "fp8bs_status_string": (_c.c_char_p, [_c.c_int]),
@@ -207,22 +212,60 @@ def _stream(index):
     return _torch()._C._cuda_getCurrentRawStream(index)
 
 
-_workspaces = {}
-_retired = []
+MAX_WORKSPACES = 16
+_workspaces = {}        # (device index, stream handle) -> tensor, oldest first
+_graph_workspaces = {}  # token -> (device index, stream handle, capture id, tensor)
+_tokens = itertools.count(1)
+_workspaces_lock = threading.Lock()
 
 
-def _workspace(device, nbytes):
-    """A zero-initialised per-device workspace, grown on demand and reused between calls."""
+def _drop_graph_workspaces():
+    """Gives up the workspaces of graphs that no longer exist."""
+    gone = (_c.c_ulonglong * 64)()
+    for i in range(lib().fp8bs_capture_released(gone, len(gone))):
+        _graph_workspaces.pop(gone[i], None)
+
+
+def _new_workspace(device, stream, nbytes):
     torch = _torch()
-    key = (device.type, device.index)
-    ws = _workspaces.get(key)
+    _drop_graph_workspaces()
+    ws = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
+    _check(lib().fp8bs_workspace_init(ws.data_ptr(), ws.numel(), stream), "fp8bs_workspace_init")
+    return ws
+
+
+def _workspace(device, index, stream, nbytes):
+    """A zero-initialised workspace for a call on the current stream of `device`: calls that may overlap on the GPU never get
+    the same one.  One per stream, grown on demand and reused between calls; a captured graph has its own, see below.  Each is
+    allocated on the stream that uses it, so one that is replaced or given up goes back to torch's allocator in stream order."""
+    if _torch().cuda.is_current_stream_capturing():
+        return _graph_workspace(device, index, stream, nbytes)
+    ws = _workspaces.get((index, stream))
     if ws is None or ws.numel() < nbytes:
-        if ws is not None:
-            _retired.append(ws)      # a captured CUDA graph may still point at the old one: keep it alive
-        ws = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _check(lib().fp8bs_workspace_init(ws.data_ptr(), ws.numel(),
-                                          torch.cuda.current_stream(device).cuda_stream), "fp8bs_workspace_init")
-        _workspaces[key] = ws
+        ws = _new_workspace(device, stream, nbytes)
+        with _workspaces_lock:
+            _workspaces.pop((index, stream), None)
+            while len(_workspaces) >= MAX_WORKSPACES:
+                del _workspaces[next(iter(_workspaces))]
+            _workspaces[(index, stream)] = ws
+    return ws
+
+
+def _graph_workspace(device, index, stream, nbytes):
+    """The workspace of a call that is being captured: one per capture and stream, zeroed by the graph itself, as graphs may be
+    replayed beside one another and beside eager calls.  Held until the graph and everything instantiated from it are gone."""
+    capture = _c.c_ulonglong(0)
+    _check(lib().fp8bs_capture_id(stream, _c.byref(capture)), "fp8bs_capture_id")
+    for owner in list(_graph_workspaces.values()):
+        if owner[:3] == (index, stream, capture.value) and owner[3].numel() >= nbytes:
+            return owner[3]
+    ws = _new_workspace(device, stream, nbytes)
+    token = next(_tokens)
+    _graph_workspaces[token] = (index, stream, capture.value, ws)
+    rc = lib().fp8bs_capture_hold(stream, token)
+    if rc != 0:
+        del _graph_workspaces[token]
+        _check(rc, "fp8bs_capture_hold")
     return ws
 
 
@@ -253,6 +296,8 @@ def gemm(A, B, a_scale, b_scale, C=None, M=None, N=None, K=None, path=PATH_AUTO,
       b_scale  float32 CUDA tensor [K/128, ceil(n_total/128)]
       C        bfloat16 CUDA tensor [M, N] (allocated if None)
     path / splits / tile_n force a kernel; n0 / n_total describe an N-shard.
+    workspace is for split-K and stream-K; without one the call uses a workspace of the current stream, or of the graph that it
+    is being captured into.  A workspace that is passed in must not be in use by another call on the GPU at the same time.
     """
     torch = _torch()
     if not A.is_cuda:
@@ -260,6 +305,7 @@ def gemm(A, B, a_scale, b_scale, C=None, M=None, N=None, K=None, path=PATH_AUTO,
     if M is None or N is None or K is None:
         raise ValueError("M, N, K are required (operands are flat column-major buffers)")
     index = A.get_device()
+    stream = _stream(index)
     if C is None:
         C = A.new_empty((M, N), dtype=torch.bfloat16)
     if n_total is None:
@@ -270,10 +316,10 @@ def gemm(A, B, a_scale, b_scale, C=None, M=None, N=None, K=None, path=PATH_AUTO,
     else:
         need = _workspace_need((index, M, N, K, path, splits, tile_n))
         if need:
-            ws = _workspace(A.device, need)
+            ws = _workspace(A.device, index, stream, need)
             ws_ptr, ws_bytes = ws.data_ptr(), ws.numel()
     rc = lib().fp8bs_gemm_ex(A.data_ptr(), B.data_ptr(), a_scale.data_ptr(), b_scale.data_ptr(), C.data_ptr(),
-                             M, N, K, n0, n_total, path, splits, tile_n, ws_ptr, ws_bytes, _stream(index))
+                             M, N, K, n0, n_total, path, splits, tile_n, ws_ptr, ws_bytes, stream)
     if rc != 0:
         _check(rc, "fp8bs_gemm_ex")
     _set_up.add(index)

@@ -809,6 +809,21 @@ static float host_e4m3fn_to_float(uint8_t b)
     return (b & 0x80) ? -v : v;
 }
 
+// fp8bs_capture_hold: a token lives in a user object of the graph.  The driver calls release_token, which must not call CUDA,
+// on a thread of its choice when the last graph that holds it is destroyed; it waits in g_released until it is asked for.
+struct HeldToken {
+    unsigned long long token;
+    HeldToken* next;
+};
+static std::atomic<HeldToken*> g_released{nullptr};
+
+static void CUDART_CB release_token(void* p)
+{
+    HeldToken* held = static_cast<HeldToken*>(p);
+    held->next = g_released.load(std::memory_order_relaxed);
+    while (!g_released.compare_exchange_weak(held->next, held, std::memory_order_release, std::memory_order_relaxed)) {}
+}
+
 constexpr int HOST_CHUNKS = 4;   // column chunks fp8bs_gemm_host pipelines (copy in, GEMM, copy out)
 
 struct fp8bs_host_ctx_impl {
@@ -960,6 +975,55 @@ int fp8bs_workspace_init(void* workspace, size_t workspace_bytes, void* stream)
     if (workspace_bytes < COUNTER_BYTES) return FP8BS_ERR_WORKSPACE;
     CUDA_TRY(cudaMemsetAsync(workspace, 0, COUNTER_BYTES, static_cast<cudaStream_t>(stream)));
     return FP8BS_OK;
+}
+
+int fp8bs_capture_id(void* stream, unsigned long long* id)
+{
+    if (!id) return FP8BS_ERR_NULL;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long capture = 0;
+    CUDA_TRY(cudaStreamGetCaptureInfo(static_cast<cudaStream_t>(stream), &status, &capture));
+    *id = status == cudaStreamCaptureStatusActive ? capture : 0;
+    return FP8BS_OK;
+}
+
+int fp8bs_capture_hold(void* stream, unsigned long long token)
+{
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    CUDA_TRY(cudaStreamGetCaptureInfo(static_cast<cudaStream_t>(stream), &status, nullptr, &graph));
+    if (status != cudaStreamCaptureStatusActive || !graph) return FP8BS_ERR_ARG;
+    HeldToken* held = new (std::nothrow) HeldToken{token, nullptr};
+    if (!held) return FP8BS_ERR_CUDA;
+    cudaUserObject_t object = nullptr;
+    const cudaError_t e = cudaUserObjectCreate(&object, held, release_token, 1, cudaUserObjectNoDestructorSync);
+    if (e != cudaSuccess) {
+        delete held;
+        CUDA_TRY(e);
+    }
+    const cudaError_t r = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
+    if (r != cudaSuccess) (void)cudaUserObjectRelease(object, 1);      // reported as released, like any other token
+    CUDA_TRY(r);
+    return FP8BS_OK;
+}
+
+int fp8bs_capture_released(unsigned long long* tokens, int max_tokens)
+{
+    if (!tokens) return 0;
+    HeldToken* list = g_released.exchange(nullptr, std::memory_order_acquire);
+    int n = 0;
+    while (list && n < max_tokens) {
+        HeldToken* next = list->next;
+        tokens[n++] = list->token;
+        delete list;
+        list = next;
+    }
+    while (list) {                                                      // no room: next time
+        HeldToken* next = list->next;
+        release_token(list);
+        list = next;
+    }
+    return n;
 }
 
 int fp8bs_last_device_status(void* stream, unsigned int* detail)

@@ -159,6 +159,15 @@ size_t fp8bs_workspace_bytes(int M, int N, int K);
 size_t fp8bs_workspace_bytes_ex(int M, int N, int K, int path, int splits, int tile_n);
 int fp8bs_workspace_init(void* workspace, size_t workspace_bytes, void* stream);
 
+/* For callers that own workspaces and whose calls may be captured into CUDA graphs, each of which needs a workspace of its
+ * own for as long as it can be replayed (the Python binding).  fp8bs_capture_id: the id of the capture that `stream` takes
+ * part in, 0 if none.  fp8bs_capture_hold: the graph being captured holds `token`.  fp8bs_capture_released: moves up to
+ * max_tokens tokens whose graphs, with everything cloned or instantiated from them, have been destroyed into `tokens` and
+ * returns their number; each is reported once.  Safe with several threads. */
+int fp8bs_capture_id(void* stream, unsigned long long* id);
+int fp8bs_capture_hold(void* stream, unsigned long long token);
+int fp8bs_capture_released(unsigned long long* tokens, int max_tokens);
+
 /* Synchronises `stream`, then returns FP8BS_OK or FP8BS_ERR_DEVICE_TIMEOUT if a kernel on
  * the current device recorded a barrier timeout since the last call (and clears the
  * record).  *detail (optional) receives the raw device status word. */
