@@ -18,7 +18,6 @@
 #include <cstdlib>
 #include <mutex>
 #include <new>
-#include <thread>
 
 namespace fp8bs {
 
@@ -1423,6 +1422,26 @@ int fp8bs_fnuz_to_fn_device(void* dst, const void* src, size_t n, unsigned int* 
     return reencode_launch(dev, dst, src, n, inexact_count, nullptr, nullptr, st);
 }
 
+// More calls at once than there are slots: the count goes through a word of device memory, and nobody waits for a slot.
+static int reencode_with_device_count(const DeviceInfo* dev, void* dst, const void* src, size_t n, unsigned int* inexact,
+                                      cudaStream_t st)
+{
+    void* count = nullptr;
+    CUDA_TRY(cudaMallocAsync(&count, sizeof(unsigned int), st));
+    unsigned int value = 0;
+    cudaError_t e = cudaMemsetAsync(count, 0, sizeof(value), st);
+    int rc = FP8BS_OK;
+    if (e == cudaSuccess) rc = reencode_launch(dev, dst, src, n, static_cast<unsigned int*>(count), nullptr, nullptr, st);
+    if (e == cudaSuccess && rc == FP8BS_OK) e = cudaMemcpyAsync(&value, count, sizeof(value), cudaMemcpyDeviceToHost, st);
+    const cudaError_t freed = cudaFreeAsync(count, st), done = cudaStreamSynchronize(st);
+    if (rc) return rc;
+    CUDA_TRY(e);
+    CUDA_TRY(freed);
+    CUDA_TRY(done);
+    *inexact = value;
+    return FP8BS_OK;
+}
+
 int fp8bs_fnuz_to_fn_device_sync(void* dst, const void* src, size_t n, unsigned int* inexact, void* stream)
 {
     if (!dst || !src || !inexact) return FP8BS_ERR_NULL;
@@ -1431,34 +1450,38 @@ int fp8bs_fnuz_to_fn_device_sync(void* dst, const void* src, size_t n, unsigned 
     int rc = device_setup(&dev);
     if (rc) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int slot = -1;
-    while (slot < 0) {                               // more callers than slots wait for one: each holds it for one kernel
-        {
-            std::lock_guard<std::mutex> lock(g_dev_mutex);
-            if (!dev->reencode_host) {
-                void *slots = nullptr, *host = nullptr, *host_dev = nullptr;
-                CUDA_TRY(cudaGetSymbolAddress(&slots, g_reencode_slots));
-                CUDA_TRY(cudaHostAlloc(&host, REENCODE_SLOTS * sizeof(unsigned int), cudaHostAllocMapped));
-                const cudaError_t e = cudaHostGetDevicePointer(&host_dev, host, 0);
-                if (e != cudaSuccess) {
-                    tl_last_cuda_error = static_cast<int>(e);
-                    (void)cudaGetLastError();
-                    (void)cudaFreeHost(host);
-                    return FP8BS_ERR_CUDA;
-                }
-                dev->reencode_slots = static_cast<ReencodeSlot*>(slots);
-                dev->reencode_host = static_cast<unsigned int*>(host);
-                dev->reencode_host_dev = static_cast<unsigned int*>(host_dev);
-            }
-            for (int i = 0; i < REENCODE_SLOTS && slot < 0; ++i)
-                if (!((dev->reencode_busy >> i) & 1ull)) slot = i;
-            if (slot >= 0) dev->reencode_busy |= 1ull << slot;
-        }
-        if (slot < 0) std::this_thread::yield();
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    CUDA_TRY(cudaStreamIsCapturing(st, &capture));
+    if (capture != cudaStreamCaptureStatusNone) {    // a result on the host cannot be captured; the capture goes on
+        tl_last_cuda_error = static_cast<int>(cudaErrorStreamCaptureUnsupported);
+        return FP8BS_ERR_CUDA;
     }
+    int slot = -1;
+    {
+        std::lock_guard<std::mutex> lock(g_dev_mutex);
+        if (!dev->reencode_host) {
+            void *slots = nullptr, *host = nullptr, *host_dev = nullptr;
+            CUDA_TRY(cudaGetSymbolAddress(&slots, g_reencode_slots));
+            CUDA_TRY(cudaHostAlloc(&host, REENCODE_SLOTS * sizeof(unsigned int), cudaHostAllocMapped));
+            const cudaError_t e = cudaHostGetDevicePointer(&host_dev, host, 0);
+            if (e != cudaSuccess) {
+                tl_last_cuda_error = static_cast<int>(e);
+                (void)cudaGetLastError();
+                (void)cudaFreeHost(host);
+                return FP8BS_ERR_CUDA;
+            }
+            dev->reencode_slots = static_cast<ReencodeSlot*>(slots);
+            dev->reencode_host = static_cast<unsigned int*>(host);
+            dev->reencode_host_dev = static_cast<unsigned int*>(host_dev);
+        }
+        for (int i = 0; i < REENCODE_SLOTS && slot < 0; ++i)
+            if (!((dev->reencode_busy >> i) & 1ull)) slot = i;
+        if (slot >= 0) dev->reencode_busy |= 1ull << slot;
+    }
+    if (slot < 0) return reencode_with_device_count(dev, dst, src, n, inexact, st);
     rc = reencode_launch(dev, dst, src, n, nullptr, dev->reencode_slots + slot, dev->reencode_host_dev + slot, st);
     const cudaError_t e = rc == FP8BS_OK ? cudaStreamSynchronize(st) : cudaSuccess;
-    if (e == cudaSuccess) *inexact = *static_cast<volatile unsigned int*>(dev->reencode_host + slot);
+    if (rc == FP8BS_OK && e == cudaSuccess) *inexact = *static_cast<volatile unsigned int*>(dev->reencode_host + slot);
     {
         // after a failed synchronisation the kernel may still be running: its slot is not given out again
         std::lock_guard<std::mutex> lock(g_dev_mutex);

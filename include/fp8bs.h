@@ -240,7 +240,8 @@ int fp8bs_fnuz_to_fn(uint8_t* dst, const uint8_t* src, size_t n, size_t* bad_ind
  * number is stored in *inexact_count (a device pointer, may be NULL).  Asynchronous on `stream`. */
 int fp8bs_fnuz_to_fn_device(void* dst, const void* src, size_t n, unsigned int* inexact_count, void* stream);
 /* The same, synchronous: returns when the stream has drained, with the number of inexact bytes in *inexact (a host word).  The
- * kernel writes the count to pinned host memory itself.  Safe with several threads and streams.  Not during stream capture. */
+ * kernel writes the count to pinned host memory itself.  Safe with several threads and streams.  On a capturing stream it
+ * returns FP8BS_ERR_CUDA without touching the capture. */
 int fp8bs_fnuz_to_fn_device_sync(void* dst, const void* src, size_t n, unsigned int* inexact, void* stream);
 
 #ifdef __cplusplus

@@ -55,3 +55,43 @@ def test_reencode_from_several_threads_and_streams():
     for t in threads:
         t.join()
     assert got == [[w] * 20 for w in want]
+
+
+def test_reencode_is_refused_under_capture_and_works_afterwards():
+    src = torch.randint(0, 256, (100000,), dtype=torch.uint8, device="cuda")
+    dst, want = f.fnuz_to_fn_device(src)
+    copy = torch.zeros_like(src)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        copy.copy_(src)
+        for _ in range(80):                                             # more often than there are slots
+            with pytest.raises(f.Fp8bsError) as error:
+                f.fnuz_to_fn_device(src, copy)
+            assert error.value.code == -7
+    graph.replay()
+    again, got = f.fnuz_to_fn_device(src)
+    assert got == want and torch.equal(again, dst) and torch.equal(copy, src)
+
+
+def test_reencode_by_more_callers_than_there_are_slots():
+    callers = 96
+    srcs = [torch.randint(0, 256, (50000 + 16 * i,), dtype=torch.uint8, device="cuda") for i in range(callers)]
+    want = [f.fnuz_to_fn_device(s) for s in srcs]
+    streams = [torch.cuda.Stream() for _ in range(24)]
+    torch.cuda.synchronize()
+    got = [None] * callers
+    together = threading.Barrier(callers)
+
+    def work(i):
+        with torch.cuda.stream(streams[i % len(streams)]):
+            together.wait(60)
+            for _ in range(5):
+                got[i] = f.fnuz_to_fn_device(srcs[i])
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(callers)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert all(g is not None and g[1] == w[1] and torch.equal(g[0], w[0]) for g, w in zip(got, want))
