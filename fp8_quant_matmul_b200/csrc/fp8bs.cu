@@ -460,7 +460,8 @@ static int check_args(int M, int N, int K, int n0, int n_total, int path, int sp
         if ((tile_n & FP8BS_SHORT_K) && ((t != 0 && t != 256) || (tile_n & (FP8BS_SPLIT_WORKSPACE | FP8BS_STREAM_K)) ||
                                          splits > 1 || path == FP8BS_PATH_MN_SMALL || K > 256))
             return FP8BS_ERR_ARG;
-        if ((tile_n & FP8BS_SMALL_M) && (tile_n != FP8BS_SMALL_M || M > SMALL_M_MAX || splits > MAX_CLUSTER_SPLITS))
+        // with or without the tile width that fp8bs_select_path reports
+        if ((tile_n & FP8BS_SMALL_M) && ((tile_n & ~128) != FP8BS_SMALL_M || M > SMALL_M_MAX || splits > MAX_CLUSTER_SPLITS))
             return FP8BS_ERR_ARG;
         if ((tile_n & FP8BS_STREAM_K) && ((tile_n & (FP8BS_TILE_PAIR | FP8BS_SPLIT_WORKSPACE)) || splits > 1 ||
                                           path == FP8BS_PATH_MN_LARGE))

@@ -2,6 +2,8 @@
 that no call is refused because the cost model now prefers a configuration with more partial sums.  Host logic only: without a
 GPU a call that passes the workspace check comes back as "no device" (-6), one that does not as -4."""
 import ctypes
+import math
+import random
 
 import pytest
 
@@ -41,3 +43,29 @@ def test_open_splits_take_what_fits(shape):
 @pytest.mark.parametrize("shape", [(1072, 6672, 896), (1136, 6480, 384), (11584, 592, 128)])
 def test_built_in_scratch_holds_some_cut_of_k(shape):
     assert small(*shape, 0, 0, static=True) == -6
+
+
+def _shapes(n, seed):
+    rng = random.Random(seed)
+
+    def size(lo, hi, step):
+        return min(hi, max(lo, int(round(math.exp(rng.uniform(math.log(lo), math.log(hi))) / step)) * step))
+
+    return [(size(16, 16384, 16), size(16, 7168, 16), size(128, 7168, 128)) for _ in range(n)]
+
+
+@pytest.mark.parametrize("shapes", [[(M, N, K) for M in range(16, 144, 16) for N in (16, 272, 7168) for K in (128, 512, 7168)],
+                                    _shapes(3000, 4)], ids=["few rows", "random"])
+def test_the_answer_of_select_path_is_accepted(shapes):
+    for shape in shapes:
+        path, splits, tile_n = f.select_path(*shape)
+        need = f.workspace_bytes(*shape)
+        assert f.workspace_bytes(*shape, path, splits, tile_n) == need, (shape, path, splits, hex(tile_n))
+        assert f.lib().fp8bs_gemm_ex(FAKE, FAKE, FAKE, FAKE, FAKE, *shape, 0, shape[1], path, splits, tile_n,
+                                     FAKE if need else None, need, None) == -6, (shape, path, splits, hex(tile_n))
+
+
+@pytest.mark.parametrize("tile_n", [256 | f.SMALL_M, 128 | f.SMALL_M | f.SHORT_K, f.SMALL_M | f.STREAM_K, f.SMALL_M | f.SPLIT_WORKSPACE,
+                                    f.SMALL_M | 64])
+def test_few_rows_combines_with_no_other_kernel(tile_n):
+    assert f.lib().fp8bs_gemm_ex(FAKE, FAKE, FAKE, FAKE, FAKE, 32, 256, 256, 0, 256, 0, 0, tile_n, None, 0, None) == -5
