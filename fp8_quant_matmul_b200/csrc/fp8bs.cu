@@ -352,7 +352,7 @@ static Config choose_config(const DeviceModel& dm, int M, int N, int K, int path
     const int want_tile = tile_n & ~(FP8BS_SPLIT_WORKSPACE | FP8BS_STREAM_K | FP8BS_SHORT_K | FP8BS_SMALL_M);
     Config best{FP8BS_PATH_MN_LARGE, 128, 1, 1, 0, 0};
     double best_cost = 1e300;
-    if (tile_n & FP8BS_SMALL_M) return small_m_config(dm, N, K, splits);
+    if (tile_n & FP8BS_SMALL_M) return small_m_config(dm, N, K, path == FP8BS_PATH_MN_LARGE ? 1 : splits);   // K is not cut there
     if (M <= SMALL_M_MAX && path == FP8BS_PATH_AUTO && splits == 0 && tile_n == 0) return small_m_config(dm, N, K, 0);
     // short K: the tile's partial sums stay in TMEM (mode 4), a member of the mn_large family (K is not cut)
     if (tile_n & FP8BS_SHORT_K) return Config{FP8BS_PATH_MN_LARGE, 256, 1, 1, 4, 0};

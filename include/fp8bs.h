@@ -69,8 +69,8 @@ extern "C" {
  * estimated fastest; OR this flag into tile_n (256 or 0) to force it (path auto or mn_large, splits 0 or 1). */
 #define FP8BS_SHORT_K        0x8000
 /* Few rows (M <= 64): 128 columns of C on the M side of the MMA, all rows of C on its N side, K cut over the 1..8 CTAs
- * of a cluster (splits, 0 = let the library choose).  Chosen by the library for such shapes when path, splits and tile_n
- * are left open; tile_n = FP8BS_SMALL_M, alone or with 128, forces it.  Needs no workspace. */
+ * of a cluster (splits, 0 = let the library choose; path mn_large: not cut).  Chosen by the library for such shapes when
+ * path, splits and tile_n are left open; tile_n = FP8BS_SMALL_M, alone or with 128, forces it.  Needs no workspace. */
 #define FP8BS_SMALL_M        0x10000
 
 /* ---- the operator ---------------------------------------------------------------- */

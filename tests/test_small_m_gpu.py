@@ -33,3 +33,13 @@ def test_few_rows_column_shard_inside_a_scale_block():
     got = run_gemm(A, shard_columns_of_B(B, N, K, n0, nl), a_s, b_s, M, nl, K, n0=n0, n_total=N)
     assert f.select_path(M, nl, K)[2] == 128 | f.SMALL_M
     assert_parity(np.ascontiguousarray(full[:, n0:n0 + nl]), got, "few rows, shard")
+
+
+def test_few_rows_on_the_path_that_does_not_cut_k():
+    M, N, K = 32, 1024, 1664
+    assert f.select_path(M, N, K)[1] > 1                                # left to itself the library cuts K
+    A, B, a_s, b_s = h.make_inputs(M, N, K, seed=79)
+    whole = run_gemm(A, B, a_s, b_s, M, N, K, splits=1, tile_n=f.SMALL_M)
+    cut = run_gemm(A, B, a_s, b_s, M, N, K, splits=4, tile_n=f.SMALL_M)
+    assert not np.array_equal(whole, cut)                               # another order of the sums: these inputs tell the two apart
+    assert np.array_equal(whole, run_gemm(A, B, a_s, b_s, M, N, K, path=f.PATH_MN_LARGE, tile_n=f.SMALL_M))
