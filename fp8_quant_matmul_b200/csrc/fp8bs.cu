@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -344,6 +345,7 @@ static double config_cost(const DeviceModel& dm, int M, int N, int K, int tile_n
 // sums through the workspace even where the cluster reduction could be used.
 // ws_limit: only configurations that need no more workspace than this (a mn_large answer to a mn_small question: there is none).
 static size_t config_workspace(int M, int N, const Config& c);
+static bool config_fits(int M, int N, const Config& c, size_t ws_limit);
 static Config choose_config(const DeviceModel& dm, int M, int N, int K, int path, int splits, int tile_n, size_t ws_limit = SIZE_MAX)
 {
     const int KB = K / 128;
@@ -377,7 +379,7 @@ static Config choose_config(const DeviceModel& dm, int M, int N, int K, int path
             if (!force_sk && tiles > dm.sm_count) continue;
             const double c = config_cost(dm, M, N, K, tn, 1, 1, 3);
             const Config cand{FP8BS_PATH_MN_SMALL, tn, 1, 1, 3, stream_k_ctas(tiles, KB, dm.sm_count)};
-            if (c < best_cost && config_workspace(M, N, cand) <= ws_limit) {
+            if (c < best_cost && config_fits(M, N, cand, ws_limit)) {
                 best_cost = c;
                 best = cand;
             }
@@ -397,7 +399,7 @@ static Config choose_config(const DeviceModel& dm, int M, int N, int K, int path
                 for (int mode = small ? 1 : 0; mode <= (cluster_ok ? 2 : (small ? 1 : 0)); ++mode) {
                     const double c = config_cost(dm, M, N, K, tn, s, cg, mode);
                     const Config cand{small ? FP8BS_PATH_MN_SMALL : FP8BS_PATH_MN_LARGE, tn, s, cg, mode, 0};
-                    if (c < best_cost && config_workspace(M, N, cand) <= ws_limit) {
+                    if (c < best_cost && config_fits(M, N, cand, ws_limit)) {
                         best_cost = c;
                         best = cand;
                     }
@@ -438,6 +440,15 @@ static size_t config_workspace(int M, int N, const Config& c)
     if (c.path != FP8BS_PATH_MN_SMALL || c.mode != 1) return 0;      // only the workspace reduction needs scratch
     const size_t half_tiles = static_cast<size_t>(ceil_div(M, 128 * c.cg)) * c.cg * ceil_div(N, c.tile_n);
     return COUNTER_BYTES + half_tiles * c.splits * (static_cast<size_t>(c.tile_n) * 128 * sizeof(float));
+}
+
+// Whether a workspace of ws_limit bytes will do for a configuration (SIZE_MAX: not asked yet, any will).
+static bool config_fits(int M, int N, const Config& c, size_t ws_limit)
+{
+    if (ws_limit == SIZE_MAX || (c.mode != 1 && c.mode != 3)) return true;
+    const size_t half_tiles = (c.mode == 3) ? static_cast<size_t>(c.ctas)
+        : static_cast<size_t>(ceil_div(M, 128 * c.cg)) * c.cg * ceil_div(N, c.tile_n);
+    return ws_limit >= config_workspace(M, N, c) && half_tiles <= COUNTER_BYTES / sizeof(unsigned int);
 }
 
 static int check_shape(int M, int N, int K)
@@ -615,10 +626,12 @@ static int launch_config(const Config& c, const TensorMaps& tm, const GemmParams
 }
 
 // `dests` / `n_dest`: null / 0 for the ordinary call (C is an M x N buffer of its own); otherwise n_dest buffers of
-// n_total columns each, all of which receive this call's columns [n0, n0 + N) (C is ignored).
+// n_total columns each, all of which receive this call's columns [n0, n0 + N) (C is ignored).  `static_scratch`: the
+// workspace is the library's own array (workspace and workspace_bytes are ignored).
 static int gemm_impl(const void* A, const void* B, const float* a_scale, const float* b_scale, void* C, int M,
                      int N, int K, int n0, int n_total, int path, int splits, int tile_n, void* workspace,
-                     size_t workspace_bytes, void* stream, void* const* dests = nullptr, int n_dest = 0)
+                     size_t workspace_bytes, void* stream, void* const* dests = nullptr, int n_dest = 0,
+                     bool static_scratch = false)
 {
     if (dests) {
         if (n_dest < 1 || n_dest > MAX_DEST) return FP8BS_ERR_ARG;
@@ -643,25 +656,38 @@ static int gemm_impl(const void* A, const void* B, const float* a_scale, const f
     const DeviceModel dm = (dev_rc == FP8BS_OK) ? dev->model : kB200Model;
     Config cfg = plan(dm, dev_rc == FP8BS_OK ? static_cast<int>(dev - g_dev) : -1, M, N, K, path, splits, tile_n);
     if (dests && cfg.mode == 2) return FP8BS_ERR_ARG;       // the cluster reduction stores C itself, to one buffer
-    const bool ws_usable = workspace && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0;
-    auto fits = [&](const Config& c) {
-        if (c.mode != 1 && c.mode != 3) return true;
-        const size_t half_tiles = (c.mode == 3) ? static_cast<size_t>(c.ctas)
-            : static_cast<size_t>(ceil_div(M, 128 * c.cg)) * c.cg * ceil_div(N, c.tile_n);
-        return ws_usable && workspace_bytes >= config_workspace(M, N, c) && half_tiles <= COUNTER_BYTES / sizeof(unsigned int);
-    };
-    if (!fits(cfg)) {
+    const size_t ws_limit = static_scratch ? STATIC_SCRATCH_BYTES
+        : (workspace && (reinterpret_cast<uintptr_t>(workspace) & 15u) == 0) ? std::min(workspace_bytes, SIZE_MAX - 1) : 0;
+    if (!config_fits(M, N, cfg, ws_limit)) {
         if (path == FP8BS_PATH_AUTO && !(tile_n & (FP8BS_STREAM_K | FP8BS_SPLIT_WORKSPACE))) {
             cfg = choose_config(dm, M, N, K, FP8BS_PATH_MN_LARGE, 1, tile_n);   // best full-K configuration
         } else {
-            // with the number of splits left open, the best way to cut K that fits: which workspace suffices does not hang on
-            // the constants of the estimate
-            if (splits != 0) return FP8BS_ERR_WORKSPACE;
-            cfg = choose_config(dm, M, N, K, path, splits, tile_n, ws_usable ? workspace_bytes : 0);
-            if (cfg.path != FP8BS_PATH_MN_SMALL || !fits(cfg)) return FP8BS_ERR_WORKSPACE;
+            // the best way to cut K as asked for that fits: which workspace suffices does not hang on the constants of the estimate
+            cfg = choose_config(dm, M, N, K, path, splits, tile_n, ws_limit);
+            if (cfg.path != FP8BS_PATH_MN_SMALL) return FP8BS_ERR_WORKSPACE;
         }
     }
     if (dev_rc) return dev_rc;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (static_scratch) {
+        // In host code the array's name is only a handle: its device address is fetched once per device, with that device current.
+        {
+            std::lock_guard<std::mutex> lock(g_dev_mutex);
+            if (!dev->static_scratch) {
+                void* ptr = nullptr;
+                const cudaError_t e = cudaGetSymbolAddress(&ptr, g_static_scratch);
+                if (e != cudaSuccess || !ptr) {
+                    tl_last_cuda_error = static_cast<int>(e);
+                    (void)cudaGetLastError();
+                    return FP8BS_ERR_CUDA;
+                }
+                dev->static_scratch = ptr;
+            }
+            workspace = dev->static_scratch;
+        }
+        // it keeps whatever the previous call left: the tile counters must start at zero
+        CUDA_TRY(cudaMemsetAsync(workspace, 0, COUNTER_BYTES, st));
+    }
 
     TensorMaps tm{};
     if ((rc = cfg.mode == 5 ? encode_few_rows_map(&tm.A, A, M, K, M <= 32 ? 32 : 64) : encode_operand_map(&tm.A, A, M, K))) return rc;
@@ -700,8 +726,6 @@ static int gemm_impl(const void* A, const void* B, const float* a_scale, const f
         g_prof_buf = prof_buf;
     }
 #endif
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
-
     if (cfg.mode == 1 || cfg.mode == 3) {
         p.counters = static_cast<unsigned int*>(workspace);
         p.partials = reinterpret_cast<float4*>(static_cast<char*>(workspace) + COUNTER_BYTES);
@@ -881,38 +905,12 @@ int fp8bs_gemm_scatter(const void* A, const void* B, const float* a_scale, const
                      stream, C_dest, n_dest);
 }
 
-// Split-K GEMM for callers that must not allocate.  The scratch is the file-scope device array above: in host code
-// its name is only a handle, so the real device address is fetched once per device with cudaGetSymbolAddress
-// (with that device current) and handed to the kernel like any caller-provided workspace.
+// Split-K GEMM for callers that must not allocate, on the file-scope device array above.
 int fp8bs_gemm_mn_small_static(const void* A, const void* B, const float* a_scale, const float* b_scale, void* C,
                                int M, int N, int K, int splits, void* stream)
 {
-    if (!A || !B || !a_scale || !b_scale || !C) return FP8BS_ERR_NULL;
-    int rc = check_args(M, N, K, 0, N, FP8BS_PATH_MN_SMALL, splits, 0);
-    if (rc) return rc;
-    // refuse anything the built-in scratch cannot hold, before touching the device
-    const Config cfg = choose_config(host_model(), M, N, K, FP8BS_PATH_MN_SMALL, splits, FP8BS_SPLIT_WORKSPACE, STATIC_SCRATCH_BYTES);
-    if (cfg.path != FP8BS_PATH_MN_SMALL || config_workspace(M, N, cfg) > STATIC_SCRATCH_BYTES) return FP8BS_ERR_WORKSPACE;
-    DeviceInfo* dev = nullptr;
-    rc = device_setup(&dev);                       // first call on a device: attribute set-up, no allocation
-    if (rc) return rc;
-    {
-        std::lock_guard<std::mutex> lock(g_dev_mutex);
-        if (!dev->static_scratch) {
-            void* ptr = nullptr;
-            const cudaError_t e = cudaGetSymbolAddress(&ptr, g_static_scratch);
-            if (e != cudaSuccess || !ptr) {
-                tl_last_cuda_error = static_cast<int>(e);
-                (void)cudaGetLastError();
-                return FP8BS_ERR_CUDA;
-            }
-            dev->static_scratch = ptr;
-        }
-    }
-    // The array keeps whatever the previous call left: the tile counters must start at zero.
-    CUDA_TRY(cudaMemsetAsync(dev->static_scratch, 0, COUNTER_BYTES, static_cast<cudaStream_t>(stream)));
-    return gemm_impl(A, B, a_scale, b_scale, C, M, N, K, 0, N, FP8BS_PATH_MN_SMALL, splits, FP8BS_SPLIT_WORKSPACE,
-                     dev->static_scratch, STATIC_SCRATCH_BYTES, stream);
+    return gemm_impl(A, B, a_scale, b_scale, C, M, N, K, 0, N, FP8BS_PATH_MN_SMALL, splits, FP8BS_SPLIT_WORKSPACE, nullptr, 0,
+                     stream, nullptr, 0, true);
 }
 
 int fp8bs_gemm_ref(const void* A, const void* B, const float* a_scale, const float* b_scale, void* C, int M, int N,

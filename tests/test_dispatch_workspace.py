@@ -1,5 +1,6 @@
-"""With the number of splits left open, a call that asks for the split-K family takes whatever cut of K its workspace holds, so
-that no call is refused because the cost model now prefers a configuration with more partial sums.  Host logic only: without a
+"""A call that asks for the split-K family takes whatever it asked for that its workspace holds, so that no call is refused
+because the cost model now prefers a configuration with more partial sums.  The built-in scratch goes through the same decision
+as a workspace of its size.  Host logic only: without a
 GPU a call that passes the workspace check comes back as "no device" (-6), one that does not as -4."""
 import ctypes
 import math
@@ -43,6 +44,28 @@ def test_open_splits_take_what_fits(shape):
 @pytest.mark.parametrize("shape", [(1072, 6672, 896), (1136, 6480, 384), (11584, 592, 128)])
 def test_built_in_scratch_holds_some_cut_of_k(shape):
     assert small(*shape, 0, 0, static=True) == -6
+
+
+@pytest.mark.parametrize("shape", [(1840, 4240, 512), (896, 9264, 128), (2144, 3680, 896)])
+def test_named_splits_take_the_tile_that_fits(shape):
+    first = f.workspace_bytes(*shape, f.PATH_MN_SMALL, 1, f.SPLIT_WORKSPACE)
+    least = min(f.workspace_bytes(*shape, f.PATH_MN_SMALL, 1, t | f.SPLIT_WORKSPACE) for t in (128, 256, 256 | f.TILE_PAIR))
+    assert least <= f.STATIC_SCRATCH_BYTES < first
+
+    def call(ws_bytes):
+        return f.lib().fp8bs_gemm_ex(FAKE, FAKE, FAKE, FAKE, FAKE, *shape, 0, shape[1], f.PATH_MN_SMALL, 1, f.SPLIT_WORKSPACE,
+                                     FAKE, ws_bytes, None)
+
+    assert call(first) == -6 and call(f.STATIC_SCRATCH_BYTES) == -6 and call(least) == -6
+    assert call(least - 1) == -4
+    assert small(*shape, 1, 0, static=True) == -6
+
+
+@pytest.mark.parametrize("ws_bytes", [1 << 40, 2 ** 64 - 1])
+def test_no_workspace_is_large_enough_for_more_tiles_than_counters(ws_bytes):
+    M, N, K = 65536, 16384, 256                               # 512 x 64 half-tiles of 256 columns, 16384 counters
+    ex = f.lib().fp8bs_gemm_ex
+    assert ex(FAKE, FAKE, FAKE, FAKE, FAKE, M, N, K, 0, N, f.PATH_MN_SMALL, 2, f.SPLIT_WORKSPACE, FAKE, ws_bytes, None) == -4
 
 
 def _shapes(n, seed):

@@ -65,6 +65,18 @@ def test_static_scratch_matches_the_workspace_entry_point(M, N, K, splits):
         assert bad == 0, "call %d vs checker: %d mismatches" % (call, bad)
 
 
+@pytest.mark.parametrize("M,N,K", [(1840, 4240, 512), (896, 9264, 128), (2144, 3680, 896)])
+def test_static_scratch_takes_named_splits_on_the_tile_that_fits(M, N, K):
+    # on the tile the library would choose with any amount of workspace the partial sums exceed the scratch
+    assert f.workspace_bytes(M, N, K, f.PATH_MN_SMALL, 1, f.SPLIT_WORKSPACE) > f.STATIC_SCRATCH_BYTES
+    (dA, dB, dAs, dBs), host = _inputs(M, N, K, seed=48)
+    got = f.gemm_mn_small_static(dA, dB, dAs, dBs, M, N, K, splits=1)
+    f.last_device_status()
+    rows = np.arange(0, M, 8, dtype=np.int32)
+    bad, first, maxerr = h.mismatches(h.oracle_gemm(*host, M, N, K, rows=rows), _bits(got)[rows])
+    assert bad == 0, "%d mismatches, first %d, max err %g" % (bad, first, maxerr)
+
+
 def test_static_scratch_is_usable_after_a_reported_timeout():
     """The wait-timeout self-test leaves a status behind; once it has been read, the built-in scratch works as before."""
     dev = torch.device("cuda:0")
