@@ -61,6 +61,16 @@ def test_named_splits_take_the_tile_that_fits(shape):
     assert small(*shape, 1, 0, static=True) == -6
 
 
+@pytest.mark.parametrize("shape", [(192, 80, 2816), (1024, 512, 7168), (352, 2000, 4992)])
+@pytest.mark.parametrize("tile_n", [0, 256, 128 | f.SPLIT_WORKSPACE, 256 | f.SPLIT_WORKSPACE, 256 | f.TILE_PAIR | f.SPLIT_WORKSPACE])
+def test_auto_dispatch_needs_no_workspace(shape, tile_n):
+    def call(splits, tile):
+        return f.lib().fp8bs_gemm_ex(FAKE, FAKE, FAKE, FAKE, FAKE, *shape, 0, shape[1], f.PATH_AUTO, splits, tile, None, 0, None)
+
+    assert call(0, tile_n) == -6 and call(1, tile_n) == -6
+    assert call(2, 128 | f.SPLIT_WORKSPACE) == -4 and call(0, 128 | f.STREAM_K) == -4       # asked for: no other path instead
+
+
 @pytest.mark.parametrize("ws_bytes", [1 << 40, 2 ** 64 - 1])
 def test_no_workspace_is_large_enough_for_more_tiles_than_counters(ws_bytes):
     M, N, K = 65536, 16384, 256                               # 512 x 64 half-tiles of 256 columns, 16384 counters
