@@ -77,8 +77,8 @@ extern "C" {
 
 /* Run-time shape dispatch between the two kernels.  Replaces the reference's manual,
  * compile-time choice (which .hip file check.cu:13 / sgemm.cu:13 includes, plus OPTION,
- * mn_large.hip:9; policy in README.md:99, 161).  Falls back to the best full-K
- * configuration if the workspace is too small for split-K. */
+ * mn_large.hip:9; policy in README.md:99, 161).  If the workspace is too small for the
+ * library's first choice, the best configuration that fits it is taken (NULL: one that needs none). */
 int fp8bs_gemm(const void* A, const void* B, const float* a_scale, const float* b_scale, void* C,
                int M, int N, int K, void* workspace, size_t workspace_bytes, void* stream);
 
@@ -90,8 +90,8 @@ int fp8bs_gemm_mn_large(const void* A, const void* B, const float* a_scale, cons
 /* Forced small-M.N / large-K path: replaces k_large_kernel<<<grid, block>>> (mn_small.hip:10;
  * launch at check.cu:92-101).  splits = 0 lets the library choose; 1 <= splits <= min(K/128, 32).
  * Partial sums are added in split order, so repeated calls give bit-identical C.  The workspace is only used
- * where fp8bs_workspace_bytes_ex reports a non-zero size for the configuration (may be NULL otherwise).  With splits = 0
- * and a workspace too small for the library's first choice, the best cut of K that fits it is taken. */
+ * where fp8bs_workspace_bytes_ex reports a non-zero size for the configuration (may be NULL otherwise).  If it
+ * is too small for the library's first choice, the best configuration with these splits that fits it is taken. */
 int fp8bs_gemm_mn_small(const void* A, const void* B, const float* a_scale, const float* b_scale,
                         void* C, int M, int N, int K, int splits, void* workspace,
                         size_t workspace_bytes, void* stream);

@@ -416,3 +416,22 @@ def test_bounded_wait_reports_a_timeout_and_leaves_the_context_usable():
     M, N, K = 128, 128, 256
     A, B, a_s, b_s = h.make_inputs(M, N, K, seed=2)
     assert_parity(h.oracle_gemm(A, B, a_s, b_s, M, N, K), run_gemm(A, B, a_s, b_s, M, N, K))
+
+
+@pytest.mark.parametrize("shape", [(352, 2000, 4992), (1488, 400, 4608), (384, 2000, 4992)])
+def test_auto_dispatch_without_a_workspace_still_cuts_k_in_a_cluster(shape):
+    M, N, K = shape
+    assert f.workspace_bytes(*shape) > 0                                # the first choice needs one
+    A, B, a_s, b_s = h.make_inputs(M, N, K, seed=31)
+    dA, dB, dAs, dBs = to_dev(A, B, a_s, b_s)
+    C = torch.empty((M, N), dtype=torch.bfloat16, device=dev())
+    assert f.lib().fp8bs_gemm(dA.data_ptr(), dB.data_ptr(), dAs.data_ptr(), dBs.data_ptr(), C.data_ptr(), M, N, K, None, 0, None) == 0
+    torch.cuda.synchronize()
+    f.last_device_status()
+    got = C.view(torch.int16).cpu().numpy().view(np.uint16)
+    rows = np.arange(0, M, 8, dtype=np.int32)
+    assert_parity(h.oracle_gemm(A, B, a_s, b_s, M, N, K, rows=rows), got[rows])
+    # partial sums are added in split order, so the bits tell how K was cut
+    whole = run_gemm(A, B, a_s, b_s, M, N, K, path=f.PATH_MN_LARGE)
+    clusters = [run_gemm(A, B, a_s, b_s, M, N, K, path=f.PATH_MN_SMALL, splits=s, tile_n=128) for s in range(2, 9)]
+    assert not np.array_equal(got, whole) and any(np.array_equal(got, c) for c in clusters)
