@@ -295,7 +295,10 @@ static int stream_k_ctas(int tiles, int KB, int sm_count)
 //   tiles; 0.4 above the fit, which settles near ties for the kernel that does not cut K), paid again with 2.8 us of
 //   prologue by every further wave of clusters;
 //   stream-K: 3.2 us per 128 columns of tile width for the hand-over of partial tiles, times half the number of CTAs that
-//   share a tile (the finishing CTA reads the others' one after the other).
+//   share a tile (the finishing CTA reads the others' one after the other), and 0.5 us above the fit, which settles near ties
+//   for the kernels that need no workspace: on 95 shapes where the fit alone has it ahead the call took up to 12 % longer than
+//   with the choice before the refit (9664 x 80 x 4608 23.7 against 21.1 us, 288 x 3152 x 5632 19.5 against 17.9), with it 7 %
+//   at most, and 4.6 % less on average (3 % without).
 // Mode 4 (K <= 256, partial sums resident in TMEM) is chosen by rule, see choose_config.
 constexpr int SHORT_K_MAX_WAVES = 3;
 static double config_cost(const DeviceModel& dm, int M, int N, int K, int tile_n, int splits, int cg, int mode)
@@ -320,7 +323,7 @@ static double config_cost(const DeviceModel& dm, int M, int N, int K, int tile_n
         // the CTA that finishes a tile reads the partial tile of every other CTA that worked on it, one after the other
         const double sharers = (kb_each < KB) ? (KB / kb_each + 1.0) : 2.0;
         return LAUNCH_US + kb_each * per_kb(g) + (static_cast<double>(tiles) / g + 1.0) * PER_UNIT[kind] +
-               3.24 * (tile_n / 128) * (sharers / 2.0);
+               3.24 * (tile_n / 128) * (sharers / 2.0) + 0.5;
     }
     const int units = tiles * splits;
     if (dm.sm_count < cg || (mode == 2 && dm.max_clusters[splits] < 1)) return 1e300;   // cannot run on this device
