@@ -86,6 +86,8 @@ def load(path):
         fn.restype = res
         fn.argtypes = args
     _lib = handle
+    _set_up.clear()     # what one build answers about a shape says nothing about another's
+    _needs.clear()
     return _lib
 
 

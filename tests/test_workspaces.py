@@ -113,3 +113,15 @@ def test_workspaces_are_given_back(box):
     box[0].gone = [first]
     call(box, 11, capture=9)
     assert set(api._graph_workspaces) == {second, box[0].held[2]}
+
+
+def test_another_build_is_asked_again(monkeypatch):
+    monkeypatch.setattr(api, "_needs", {})
+    monkeypatch.setattr(api, "_set_up", {0})
+    monkeypatch.setattr(api, "_lib", None)
+    key = (0, 1024, 512, 7168, f.PATH_MN_SMALL, 3, 128 | f.SPLIT_WORKSPACE)
+    need = api._workspace_need(key)
+    api._set_up.add(0)
+    assert need > 0 and api._workspace_need(key) == need and api._needs == {key: need}
+    api.load(api._LIB_PATH)
+    assert not api._needs and not api._set_up
