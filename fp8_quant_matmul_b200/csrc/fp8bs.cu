@@ -242,8 +242,6 @@ constexpr int MAX_CLUSTER_SPLITS = 8;   // portable cluster size limit; 7 and 8 
 
 static inline int ceil_div(int a, int b) { return (a + b - 1) / b; }
 
-// Stream-K grid: every SM, but at least 4 K blocks per CTA.  Never more CTAs than SMs: a CTA waits (bounded) for
-// partial tiles of CTAs that must therefore be running at the same time.
 constexpr int SMALL_M_MAX = 64;
 
 // Mode 5: K is cut over as many CTAs as there are SMs to read B with (tiles are 128 columns wide).  Measured with 1, 2, 3, ..
@@ -266,6 +264,8 @@ static Config small_m_config(const DeviceModel& dm, int N, int K, int splits)
     return Config{s > 1 ? FP8BS_PATH_MN_SMALL : FP8BS_PATH_MN_LARGE, 128, s, 1, 5, 0};
 }
 
+// Stream-K grid: every SM, but at least 4 K blocks per CTA.  Never more CTAs than SMs: a CTA waits (bounded) for
+// partial tiles of CTAs that must therefore be running at the same time.
 static int stream_k_ctas(int tiles, int KB, int sm_count)
 {
     const long long total = static_cast<long long>(tiles) * KB;
@@ -279,11 +279,13 @@ static int stream_k_ctas(int tiles, int KB, int sm_count)
 // Estimated run time of a configuration in microseconds.  The constants are a least-squares fit to a sweep of every
 // configuration over 94 shapes on a B200 (the 18 benchmark shapes, random and ragged ones, M 80..16384, N 64..7168, K 128..7168,
 // cold L2, launches back to back); choosing by it costs 0.3 % on average against the best configuration of each shape, 6 % at
-// most.  A 128-K block of a work unit takes the larger of two times:
+// most, of these 94; elsewhere up to 15 % was seen (944 x 1360 x 6272: pairs with K cut in three, 21.1 us, passed over for 25.1).
+// A 128-K block of a work unit takes the larger of two times:
 //   its MMAs, promotion and hand-over: 0.24 us (128-wide tile), 0.46 (256-wide), 0.37 (256 x 256 pair), and up to 22 / 10 / 7 %
 //   more the more SMs take part;
 //   its loads: 0.24 / 0.34 / 0.25 us, and 91 % more where the rows of an operand's boxes do not start on 32-byte sectors
-//   (M or N an odd multiple of 16: 1968 x 496 x 7040 takes 32.4 us on 128-wide tiles, 2048 x 512 x 7168 17.5).
+//   (M or N an odd multiple of 16: 1968 x 496 x 7040 takes 32.4 us on 128-wide tiles, 2048 x 512 x 7168 17.5).  A fitted
+//   factor: that such a row touches five sectors instead of four explains 25 % of it, the rest is not explained.
 // Per work unit 1.9 / 2.0 / 2.4 us (tile switch, epilogue), 1.9 us per launch.
 // Examples, 128-wide / 256-wide / pair: 1024 x 7168 x 2304 23.1 / 22.9 / 20.0 us, 128 x 7168 x 2304 9.2 / 13.3 / 11.8, 1024 x
 // 1536 x 7168 18.7 / 28.0 / 23.9 (best with K cut: 20.7).
@@ -362,12 +364,16 @@ static Config choose_config(const DeviceModel& dm, int M, int N, int K, int path
     // short K: the tile's partial sums stay in TMEM (mode 4), a member of the mn_large family (K is not cut)
     if (tile_n & FP8BS_SHORT_K) return Config{FP8BS_PATH_MN_LARGE, 256, 1, 1, 4, 0};
     if (KB <= 2 && path != FP8BS_PATH_MN_SMALL && splits <= 1 && !force_ws && !force_sk && want_tile == 0) {
-        // 256-wide single-CTA tiles, the answer fp8bs_select_path has always given for such K (with many tiles the pair is
-        // 7-9 % ahead: 6144 x 7168 x 256 18.8 us).  Of their two kernels, on a B200, this one is 1-7 % faster than the full-K
-        // kernel with few tiles per SM (1104 x 3344 x 256 5.61 against 5.88 us, 2144 x 112 x 128 3.81 against 4.05, 1024 x
-        // 7168 x 256 7.00 against 7.02); with more the store path of the SMs sets the pace and the full-K kernel, which
-        // overlaps the MMAs of a tile with the scaling of the one before, is ahead (2528 x 4496 x 256, 2.4 per SM: 9.06
-        // against 9.70; 6144 x 7168 x 256, 9.1: 20.7 against 22.2).
+        // 256-wide single-CTA tiles, by rule and not by the estimate.  Where the estimate before the refit took 128-wide ones (K
+        // = 256, more than three tiles per SM) they are ahead (2048 x 7168 x 256 9.87 against 10.14 us, 16384 x 1552 x 256 16.8
+        // against 17.5) unless half a tile is padding (32768 x 384 x 256 10.2 against 9.9). Of their two kernels this one is
+        // ahead by up to 4 %, or level, up to about 1.8 tiles per SM (1104 x 3344 x 256, 0.85: 5.67 against 5.86 us; 1024 x 7168
+        // x 256, 1.5: 7.01 and 6.98; 11600 x 736 x 256, 1.8: 7.35 and 7.33) and behind from there on, where the full-K kernel
+        // overlaps the MMAs of a tile with the scaling of the one before (2528 x 4496 x 256, 2.4: 10.1 against 9.1; 1536 x 9472
+        // x 256, 3.0: 10.1 against 8.8; 6144 x 7168 x 256, 9.1: 22.7 against 20.6).  The line still lies at three, where the two
+        // met before the full-K kernel handed its tiles over in two parts.  Known to be ahead and not taken: the pair with more
+        // than three tiles per SM (3072 x 7168 x 256 11.9 against 12.8, 9568 x 2800 x 256 14.9 against 18.1, 6144 x 7168 x 256
+        // 20.1 against 20.6), 128-wide tiles at K = 128 (2528 x 4496 7.3 against 7.95, 6144 x 7168 18.2 against 18.8).
         const int tiles = ceil_div(M, 128) * ceil_div(N, 256);
         return Config{FP8BS_PATH_MN_LARGE, 256, 1, 1, (KB == 1 || tiles <= SHORT_K_MAX_WAVES * dm.sm_count) ? 4 : 0, 0};
     }
@@ -1163,7 +1169,7 @@ int fp8bs_host_ctx_create(fp8bs_host_ctx** out, size_t max_M, size_t max_N, size
     std::memset(c, 0, sizeof(*c));
     c->max_M = max_M; c->max_N = max_N; c->max_K = max_K;
     const size_t KB = max_K / 128;
-    // split-K is only ever chosen for small M*N; 64 MiB covers every such configuration
+    // what the dispatch wants for M, N, K up to 8192 is below this; beyond, it takes the best configuration that fits
     c->w_bytes = static_cast<size_t>(64) << 20;
     bool ok = cudaMalloc(&c->dA, max_M * max_K) == cudaSuccess && cudaMalloc(&c->dB, max_N * max_K) == cudaSuccess &&
               cudaMalloc(&c->dAs, max_M * KB * 4) == cudaSuccess && cudaMalloc(&c->dBs, BSCALE_MAX_BYTES) == cudaSuccess &&

@@ -242,11 +242,6 @@ struct FloatCols {
     __device__ __forceinline__ uint32_t bf16_pair(int i) const { return pack_bf16x2(v[2 * i], v[2 * i + 1]); }
 };
 
-// Converts 64 columns of this thread's row to bf16 (round to nearest even) into a 32-row x 128-byte staging
-// box laid out as the 128-byte-swizzled TMA store expects; then one lane issues the store.
-// The box covers rows [row0, row0 + 32) and columns [col, col + 64); lane = row within the box.
-// PENDING: how many of this thread's most recent stores may still be reading shared memory (1 when the warp
-// alternates between two boxes: only the store before the last one used this box); negative: the caller has waited.
 // Converts 64 columns of this thread's row to bf16 (round to nearest even) into row `lane` of a 32-row x 128-byte
 // staging box, laid out as the 128-byte-swizzled TMA store expects.
 template <class Cols>
@@ -264,6 +259,8 @@ __device__ __forceinline__ void stage_64(uint8_t* stg, int lane, const Cols cols
     }
 }
 
+// stage_64, then one lane issues the store of the box, which covers rows [row0, row0 + 32) and columns [col, col + 64).
+// PENDING: how many of this warp's most recent stores may still be reading shared memory; negative: the caller has waited.
 template <int PENDING, class Cols>
 __device__ __forceinline__ void stage_and_store_64(const CUtensorMap* tmC, int n_dest, uint8_t* stg, uint32_t stg_addr,
                                                    int lane, const Cols cols, int col, int row0, int M, int N)

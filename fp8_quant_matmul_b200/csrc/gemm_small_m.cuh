@@ -14,7 +14,7 @@
 // All waits are bounded as there.
 //
 // Measured on a B200 (CUDA graph, cold weights), 128-row tiles -> this kernel: 16 x 7168 x 2304 14.9 -> 7.9 us, 32 x 4096 x 2048
-// 8.7 -> 5.8, 64 x 7168 x 2304 10.7 -> 9.4, 16 x 1536 x 7168 10.8 -> 6.1, 16 x 7168 x 7168 20.9 -> 16.1 (the weights alone take 2.5,
+// 8.7 -> 5.8, 64 x 7168 x 2304 10.7 -> 9.4, 16 x 1536 x 7168 10.8 -> 6.1, 16 x 7168 x 7168 20.9 -> 14.0 (the weights alone take 2.5,
 // 1.3, 2.5, 1.7 and 7.7 us at 6.65 TB/s); the smallest call, 16 x 128 x 128, 3.1 -> 2.3.
 #pragma once
 #include "gemm_kernel.cuh"
